@@ -278,3 +278,89 @@ def tolerance(case):
     # and by at most 3.1e-3 of their root mean square (tensor-core and one-token paths alike); four times that is stated.
     # Where the hidden state is part of the output it hides some of the difference.  Expert ids are whole: none may differ.
     return {"rel": 1.7e-3, "max": 1.2e-2}
+
+
+# ── the same in 64 bits ──────────────────────────────────────────────────────────────────────
+
+PAGE_BYTES = 2 << 20
+
+
+def _matrix64(model, layer, expert, segment):
+    """One INT4 matrix of the pool as float64: per page [rows x K/2] code bytes (low nibble = even column, weight =
+    (nibble - 8) * scale), then [rows x K/32] fp16 scales."""
+    store, parts = model.pool.storage, []
+    for pg in sorted((p for p in model.by_expert[layer, expert] if p.pid.segment == segment), key=lambda p: p.row_start):
+        raw, n = store[pg.slot * PAGE_BYTES:(pg.slot + 1) * PAGE_BYTES], pg.row_count * pg.cols // 2
+        codes = raw[:n].view(pg.row_count, pg.cols // 2)
+        scales = raw[n:n + pg.row_count * pg.cols // 16].clone().view(torch.float16).view(pg.row_count, pg.cols // 32)
+        w = torch.stack((codes & 15, codes >> 4), dim=2).view(pg.row_count, pg.cols).double() - 8.0
+        parts.append((w.view(pg.row_count, -1, 32) * scales.double()[:, :, None]).view(pg.row_count, pg.cols))
+    return torch.cat(parts)
+
+
+def _experts64(model, layer, x, pairs, shared_tokens):
+    """Sum over a token's experts of weight * down(silu(gate x) * up x); pairs: [(token, expert, weight)]."""
+    out = torch.zeros_like(x)
+    by_expert = {}
+    for t, e, w in pairs:
+        by_expert.setdefault((e, 0), []).append((t, w))
+    if shared_tokens:
+        by_expert[0xFFFF, 14] = [(t, 1.0) for t in shared_tokens]     # (the shared expert's segments are 14, 15, 16)
+    for (e, seg), use in by_expert.items():
+        rows = torch.tensor([t for t, _ in use], device=x.device)
+        xe = x[rows]
+        act = torch.nn.functional.silu(xe @ _matrix64(model, layer, e, seg + 1).T) * (xe @ _matrix64(model, layer, e, seg).T)
+        y = act @ _matrix64(model, layer, e, seg + 2).T
+        out.index_add_(0, rows, y * torch.tensor([w for _, w in use], device=x.device, dtype=torch.float64)[:, None])
+    return out
+
+
+def _route64(sh, x, w, offset, bias):
+    logits = x @ w.double().T
+    if offset is not None:
+        logits = logits + offset.double()
+    if sh.scoring == SCORING_SOFTMAX:
+        top, ids = torch.topk(logits, sh.top_k, dim=1)
+        return ids, torch.softmax(top, dim=1)
+    score = torch.sigmoid(logits)
+    ids = torch.topk(score if bias is None else score + bias.double(), sh.top_k, dim=1).indices
+    wt = score.gather(1, ids)
+    return ids, wt / wt.sum(1, keepdim=True) * sh.scaling_factor
+
+
+def exact(case, seed):
+    """What run returns, in 64 bits from the dequantised pages; expert ids, which are whole numbers, are left out."""
+    s = prepare(case, seed)
+    kind, sh, L, T, model = s["kind"], s["sh"], s["L"], s["T"], s["model"]
+    (lo, hi), outs, weights = s["range"], [], None
+    model.by_expert = {}
+    for p in model.pages:
+        model.by_expert.setdefault((p.pid.layer, p.pid.expert), []).append(p)
+    for l in range(L):
+        x, h = s["xs"][l].double(), None
+        if kind == "stack":
+            h = s["h0"][l].double() + s["attn"][l].double()
+            # (the sublayer's input is rounded to its activation type on the way)
+            x = (h / torch.sqrt((h * h).mean(1, keepdim=True) + 1e-6) * s["norm"][l].double()).to(s["x"].dtype).double()
+        if kind == "ep_pairs":
+            ids, wt = s["ids"][l][:, :sh.top_k].long(), s["w"][l][:, :sh.top_k].double()
+        else:
+            ids, wt = _route64(sh, x, s["w16"][0] if kind == "paged" else model.router_w[l], s["offset"], s["bias"])
+        weights = wt
+        pairs = [(t, e, w) for t, (es, ws) in enumerate(zip(ids.tolist(), wt.tolist())) for e, w in zip(es, ws) if lo <= e < hi]
+        shared = [] if not sh.shared_experts or kind == "ep_share" else [1] if kind == "ep_pairs" else range(T)
+        out = _experts64(model, l, x, pairs, shared)
+        outs.append(out if h is None else h + out)
+    if kind == "step_host":
+        return [o[0].cpu() for o in outs]
+    if kind == "layer":
+        return torch.cat(outs), None
+    if kind in ("stack", "ep_pairs"):
+        return torch.stack(outs)
+    if kind == "tokens":
+        full = torch.zeros(T, s["gd"].weights.shape[1], dtype=torch.float64, device=x.device)
+        full[:, :sh.top_k] = weights
+        return outs[0], None, full
+    if kind == "ep_share":
+        return outs[0], None
+    return outs[0][0], None, weights[0].cpu().numpy()
