@@ -104,3 +104,28 @@ def test_grouped_accumulates_and_refuses_bad_arguments(cuda_dev):
     assert int(gd.status.item()) == 0
     assert torch.allclose(part, whole, rtol=0, atol=2e-5)
     assert lib().vib3_moe_grouped_workspace_bytes(0, 8, 384, 7168, 2048, 520, 1820) == 0
+
+
+@pytest.mark.parametrize("H,I", [(768, 256), (256, 1280), (2304, 512)])
+def test_token_counts_and_slab_counts_at_the_edges(cuda_dev, oracle, H, I):
+    """Every token chooses every expert, so an expert has T tokens: the accumulator widths (4, 8, 16), one and two token
+    groups and several passes, over odd, single and partial slab counts of both projections."""
+    from vic_b200.core_types import SCORING_SOFTMAX, MoeShape
+    from vic_b200.grouped import GroupedDecoder
+    from vic_b200.synth import build_synthetic_moe, synth_activation
+    sh = MoeShape("grp-edges", H, I, 3, 3, 0, SCORING_SOFTMAX, 1.0, True)
+    model = build_synthetic_moe(sh, 1, cuda_dev, seed=H + I, slot_seed=5)
+    gd = GroupedDecoder(model, max_tokens=97)
+    g = torch.Generator(device=cuda_dev).manual_seed(H)
+    xs = synth_activation(sh, g, cuda_dev, torch.float16, 97)
+    xs_n = xs.float().cpu().numpy()
+    want = None
+    for T in (97, 2, 4, 5, 8, 9, 16, 17, 24, 32, 33, 49, 64):
+        out = gd.forward(0, xs[:T]).cpu().numpy()
+        assert int(gd.status.item()) == 0
+        if want is None:
+            ids, ws = gd.ids[:T, :3].cpu().numpy().view(np.uint16), gd.weights[:T, :3].cpu().numpy()
+            want = [oracle.moe_layer(xs_n[t], oracle_experts(oracle, model, 0, list(zip(ids[t].tolist(), ws[t].tolist()))), H, I,
+                                     oracle.SCALE_FP16, "gpu") for t in range(T)]
+        for t in range(T):
+            assert_close(out[t], want[t], f"T={T} token {t}")

@@ -8,23 +8,25 @@
 //   D[128 weight rows x N tokens] += A[128 x 256] . B[N x 256]^T      per 256-column slab of K
 //
 //   A  the INT4 page tile.  cp.async.bulk.tensor (one 3-D tensor map over the whole page pool: byte in
-//      row, row in page, pool slot) brings 128 B of codes per row and slab — and, once per tile, the rows' group
-//      scales for all of K: the TMA unit pays per row segment, so 16-byte scale segments per slab would cost as
-//      much as the codes — into shared
-//      memory (128-byte swizzle, so that 32 lanes reading 32 rows hit 32 different bank groups); eight
-//      warps turn the codes into fp16 weights (n - 8) * scale in registers and store them with tcgen05.st
-//      into TENSOR MEMORY: the A operand never goes back through shared memory, whose bandwidth could
-//      not carry 4x-expanded weights at the HBM rate.
+//      row, row in page, pool slot) brings 128 B of codes per row and slab, and the rows' group scales for four
+//      slabs at a time (64 bytes of a row: a 16-byte piece per slab would cost half a memory sector and a row
+//      segment of the TMA unit each), into shared memory (swizzled, so that lanes reading consecutive rows hit
+//      different banks).  Converting warps turn the codes into the whole numbers n - 8 as fp16, exactly, and store
+//      them with tcgen05.st into TENSOR MEMORY: the A operand never goes back through shared memory, whose
+//      bandwidth could not carry 4x-expanded weights at the HBM rate.
 //   B  the tokens of the expert: rows of a gathered fp16 activation matrix (pairs sorted by expert), loaded
 //      by the same TMA unit as 128-byte-swizzled K-major tiles and read by the MMA through a shared-memory
 //      descriptor.  Within every 8 columns the K order of both operands is (0,4,1,5,2,6,3,7): that is
 //      the order in which one logic operation per two weights isolates the 4-bit codes, and a contraction
 //      does not care about the order of K as long as both operands agree.
-//   D  fp32 in tensor memory; tcgen05.ld brings it to registers for the epilogue (gate/up: SiLU product
-//      rounded to fp16 as the batch-1 path does; down: fp16 per (pair, row), combined per token in plan
-//      order by a last kernel, so that the result does not depend on scheduling).
+//   D  fp32 in tensor memory, one accumulator per scale group of 32 columns (two MMAs of 16): scaling warps read a
+//      slab's accumulators with tcgen05.ld and add scale * D to their fp32 sums in registers, packed fp32 FMAs over
+//      as many token columns as the expert has (4, 8 or 16).  The scale costs one FMA per 32 weights and token
+//      instead of one product per weight, and nothing is rounded between the codes and the fp32 sums.
+//      At the end of a tile: gate/up SiLU product rounded to fp16 as the batch-1 path does; down fp16 per (pair, row),
+//      combined per token in plan order by a last kernel, so that the result does not depend on scheduling.
 //
-// One elected thread issues the MMAs; completion is tracked with tcgen05.commit on mbarriers.  Every wait is
+// One elected thread per issuing warp issues MMAs; completion is tracked with tcgen05.commit on mbarriers.  Every wait is
 // bounded: a thread that gives up sets VIB3_STATUS_TIMEOUT and the CTA drains and frees its tensor memory.
 // No cluster launch, no multicast: every CTA fetches its own tiles.
 //
@@ -43,26 +45,27 @@
 
 namespace vib3 {
 
-constexpr int kGrpConvWarps = 16;               // converting warps: two teams of 8; TMEM lane quarter = warp & 3
-constexpr int kGrpMmaWarps = 4;                 // MMA-issuing warps: a thread issues one tcgen05.mma per ~100 cycles whatever its
-                                                // size (measured), four issuers reach the tensor pipe's own rate
-constexpr int kGrpFirstEpiWarp = 1 + kGrpMmaWarps;          // warp 0 TMA, 1..4 MMA, 5..8 epilogue, 9..24 converting
-constexpr int kGrpFirstConvWarp = kGrpFirstEpiWarp + 4;
-constexpr int kGrpXWarp = kGrpFirstConvWarp + kGrpConvWarps;   // issues the token tiles' copies
-constexpr int kGrpThreads = (kGrpXWarp + 1) * 32;
-constexpr int kGrpStages = 8;                   // weight ring
+// Warp roles: 0 weights' copies, 1 tokens' copies, 2.. MMA issuers, then scaling and converting warps.
+constexpr int kGrpXWarp = 1, kGrpMmaWarp = 2;
+constexpr int kGrpMmaWarps = 4;                 // an issuing warp takes every fourth scale group's MMAs
+constexpr int kGrpFirstScaleWarp = kGrpMmaWarp + kGrpMmaWarps;   // two teams of four; TMEM lane quarter = warp & 3
+constexpr int kGrpFirstConvWarp = kGrpFirstScaleWarp + 8;        // two teams of four
+constexpr int kGrpThreads = (kGrpFirstConvWarp + 8) * 32;
 constexpr int kGrpSlabK = 256;                  // columns of K per pipeline step
-constexpr int kGrpMaxN = 16;                    // tokens of one expert per accumulator (a "pass"); a slab is converted once for
-                                                // up to TWO passes: the second token group goes to the other D buffer
-constexpr int kGrpABufs = 3;                    // A-operand buffers in tensor memory: the converting warps run up to two slabs ahead
-constexpr int kGrpXStages = kGrpABufs;          // token ring: stage i is released together with A buffer i (one commit frees both)
-constexpr int kGrpRawBytes = 18 * 1024;         // a weight stage: codes 16 KB + scales 2 KB of 128 rows x 256 columns
-constexpr int kGrpXGroupBytes = kGrpMaxN * kGrpSlabK * 2;   // 16 tokens x 256 columns fp16 = 8 KB
-constexpr int kGrpXBytes = 2 * kGrpXGroupBytes;         // a token stage: the two token groups of a double pass
+constexpr int kGrpMaxN = 16;                    // tokens of one expert per token group; a slab is converted once for up to two groups
+constexpr int kGrpStages = 8;                   // code ring
+constexpr int kGrpCodeBytes = 16 * 1024;        // codes of 128 rows x 256 columns
+constexpr int kGrpXStages = 6;                  // token ring: one token group and slab per stage
+constexpr int kGrpXBytes = kGrpMaxN * kGrpSlabK * 2;   // 16 tokens x 256 columns fp16
+constexpr int kGrpChunkSlabs = 4;               // slabs whose scales travel together: 64 bytes of a row per copy
+constexpr int kGrpScaleStages = 3;              // scale ring
+constexpr int kGrpScaleBytes = 128 * kGrpChunkSlabs * 16;
 constexpr int kGrpTmemCols = 512;
-constexpr int kGrpACols = kGrpSlabK / 2;        // 128 columns: 256 fp16 per row
-constexpr int kGrpDCol0 = kGrpABufs * kGrpACols;   // the A buffers, then two D buffers of kGrpMmaWarps partial accumulators of kGrpMaxN columns
-static_assert(kGrpDCol0 + 2 * kGrpMmaWarps * kGrpMaxN <= kGrpTmemCols, "tensor memory budget");
+constexpr int kGrpACols = kGrpSlabK / 2;        // an A buffer: 256 fp16 per row
+constexpr int kGrpDCols = 8 * kGrpMaxN;         // an accumulator buffer: 8 scale groups x 16 tokens
+constexpr int kGrpDCol0 = 2 * kGrpACols;
+static_assert(kGrpDCol0 + 2 * kGrpDCols <= kGrpTmemCols, "tensor memory budget");
+static_assert(kGrpStages % 2 == 0, "the uses of a code stage belong to one converting team");
 constexpr int kGrpMaxTokens = 128;
 constexpr int kRouterMaxExpertsGrouped = 512;   // MAX_EXPERTS, src/core/types.rs:20
 
@@ -79,8 +82,8 @@ struct GroupedWork {
 };
 
 struct Unit;
-// Trips over a unit's slabs: its passes are taken two at a time (each converted slab feeds both).
-__host__ __device__ constexpr int grp_double_passes(int n_tok) { return (n_tok + 2 * kGrpMaxN - 1) / (2 * kGrpMaxN); }
+// Trips over a unit's slabs: one per 32 tokens.
+__host__ __device__ constexpr int grp_passes(int n_tok) { return (n_tok + 2 * kGrpMaxN - 1) / (2 * kGrpMaxN); }
 struct GroupedArgs {
     const GroupedWork* work;
     __half* act;             // [pairs][I], K order permuted
@@ -92,37 +95,57 @@ struct GroupedArgs {
     int* status;
 };
 
-// The waits of this kernel: mbarrier.try_wait with a suspend-time hint, so that a waiting warp sleeps in hardware
-// until the barrier's phase completes (or the hint runs out) instead of polling.  Bounded: kGrpWaitTries tries of kGrpWaitHintNs each
-// (about four seconds), then false.
-constexpr unsigned kGrpWaitHintNs = 4000000u;
-constexpr unsigned kGrpWaitTries = 1024u;
-__device__ __forceinline__ bool mbar_wait_hint(uint64_t* bar, unsigned parity) {
-    const uint32_t addr = smem_u32(bar);
-    for (unsigned it = 0; it < kGrpWaitTries; ++it) {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok) : "r"(addr), "r"(parity), "r"(kGrpWaitHintNs) : "memory");
-        if (ok) return true;
-    }
-    return false;
+// An mbarrier of this kernel by its 32-bit shared-memory address; `+ i` is the i-th of an array.
+struct Bar {
+    uint32_t addr;
+    __device__ __forceinline__ Bar operator+(int i) const { return Bar{addr + 8u * (uint32_t)i}; }
+};
+// The waits of this kernel: one look that does not suspend the warp, then suspending tries without a time limit of their
+// own.  A try with a suspend-time hint resumed later: with the hint the 32-token Kimi layer took 1025 us, without 983.
+// Bounded like every wait here; false when it gave up.
+__device__ __forceinline__ bool mbar_wait_grp(Bar bar, unsigned parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar.addr), "r"(parity) : "memory");
+    for (unsigned it = 0; !ok && it < kSpinLimit; ++it)
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"(bar.addr), "r"(parity) : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ void mbar_init(Bar bar, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar.addr), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(Bar bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar.addr), "r"(bytes) : "memory");
+}
+// one arrival for the warp (predicated, no branch)
+__device__ __forceinline__ void mbar_arrive_lane0(Bar bar, int lane) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar.addr), "r"(lane) : "memory");
 }
 
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, Bar bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-                 ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)) : "memory");
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar.addr) : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+// One lane of the warp, the same one every time.  MMAs and tensor copies take their operands from uniform registers:
+// behind elect.sync, with operands that are uniform by construction, they issue back to back; behind `lane == 0` each of
+// their operands is moved over one by one.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ void umma_commit(Bar bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar.addr) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// 32 codes (one scale group, word j = columns 8j .. 8j+7) -> 16 half2 of (n - 8) * scale in the K order
+// 32 codes (one scale group, word j = columns 8j .. 8j+7) -> 16 half2 of n - 8 in the K order
 // (0,4),(1,5),(2,6),(3,7) per word.  (n + 1024) and (16 n + 1024) are exact fp16 numbers made by one logic
-// operation per pair; subtracting 1032, or multiplying by 1/16 and subtracting 72, is exact as well; the
-// only rounding is the product with the scale.
-__device__ __forceinline__ void dequant_chunk(const uint4& q, uint32_t scale2, uint32_t* out) {
+// operation per pair; subtracting 1032, or multiplying by 1/16 and subtracting 72, is exact as well.
+__device__ __forceinline__ void codes_to_f16(const uint4& q, uint32_t* out) {
     const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -131,28 +154,74 @@ __device__ __forceinline__ void dequant_chunk(const uint4& q, uint32_t scale2, u
         const uint32_t a1 = lop3_and_or(w[j], 0x00F000F0u, 0x64006400u);
         const uint32_t a2 = lop3_and_or(w8, 0x000F000Fu, 0x64006400u);
         const uint32_t a3 = lop3_and_or(w8, 0x00F000F0u, 0x64006400u);
-        uint32_t r0, r1, r2, r3;
-        asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r0) : "r"(a0), "r"(0x64086408u));                  // (n + 1024) - 1032
-        asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r1) : "r"(a1), "r"(0x2C002C00u), "r"(0xD480D480u));  // / 16 - 72
-        asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r2) : "r"(a2), "r"(0x64086408u));
-        asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r3) : "r"(a3), "r"(0x2C002C00u), "r"(0xD480D480u));
-        asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(out[4 * j + 0]) : "r"(r0), "r"(scale2));
-        asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(out[4 * j + 1]) : "r"(r1), "r"(scale2));
-        asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(out[4 * j + 2]) : "r"(r2), "r"(scale2));
-        asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(out[4 * j + 3]) : "r"(r3), "r"(scale2));
+        asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(out[4 * j + 0]) : "r"(a0), "r"(0x64086408u));                       // (n + 1024) - 1032
+        asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(out[4 * j + 1]) : "r"(a1), "r"(0x2C002C00u), "r"(0xD480D480u));  // / 16 - 72
+        asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(out[4 * j + 2]) : "r"(a2), "r"(0x64086408u));
+        asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(out[4 * j + 3]) : "r"(a3), "r"(0x2C002C00u), "r"(0xD480D480u));
     }
 }
 
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
                  ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-                 "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+                 "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]),
+                 "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
 }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-                   "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr) : "memory");
+// N columns of this lane's row (N = 4, 8, 16); the values are there after tmem_ld_wait.
+template <int N>
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t* r) {
+    if constexpr (N == 4)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+    else if constexpr (N == 8)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+    else
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                       "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                     : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// acc[t] += scale * D[group][t] for the eight groups of a slab and NE tokens (packed pairs of fp32 FMAs): the accumulators
+// hold integer-weight sums over 32 columns, the scale of the group is applied here in fp32.  `release` is arrived on
+// once the accumulators are in registers.
+template <int NE>
+__device__ __forceinline__ void scale_slab(uint32_t taddr, const uint4& sc, float2* acc, Bar release, int lane) {
+    constexpr int kBatch = NE == 4 ? 8 : NE == 8 ? 4 : 2;   // groups read together: 32 registers
+    const uint32_t sw[4] = {sc.x, sc.y, sc.z, sc.w};
+#pragma unroll
+    for (int g0 = 0; g0 < 8; g0 += kBatch) {
+        uint32_t d[kBatch][NE];
+#pragma unroll
+        for (int g = 0; g < kBatch; ++g) tmem_ld<NE>(taddr + (g0 + g) * kGrpMaxN, d[g]);
+        tmem_ld_wait();
+        if (g0 + kBatch == 8) {
+            tc_fence_before();
+            __syncwarp();
+            mbar_arrive_lane0(release, lane);
+        }
+#pragma unroll
+        for (int g = 0; g < kBatch; ++g) {
+            const uint32_t pair = sw[(g0 + g) >> 1];
+            const float s = __half2float(__ushort_as_half((unsigned short)((g0 + g) & 1 ? pair >> 16 : pair & 0xFFFFu)));
+            uint64_t s2;
+            asm("mov.b64 %0, {%1, %1};" : "=l"(s2) : "f"(s));
+#pragma unroll
+            for (int j = 0; j < NE / 2; ++j) {
+                uint64_t dv, av;
+                asm("mov.b64 %0, {%1, %2};" : "=l"(dv) : "r"(d[g][2 * j]), "r"(d[g][2 * j + 1]));
+                asm("mov.b64 %0, {%1, %2};" : "=l"(av) : "f"(acc[j].x), "f"(acc[j].y));
+                asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(av) : "l"(dv), "l"(s2));
+                asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[j].x), "=f"(acc[j].y) : "l"(av));
+            }
+        }
+    }
+}
+
+__device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                 ::"r"(d), "r"(a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
 // Position of row r (column of the down projection) in the permuted K order.
@@ -178,30 +247,22 @@ static_assert(sizeof(Unit) == 32, "a unit is two 16-byte loads");
 struct UnitWalk {
     const Unit* units;
     int n_units, u;
-    Unit cur, nxt;
-    bool have_next;
-    __device__ __forceinline__ void load(Unit& t, int i) const {
-        const uint4* p = reinterpret_cast<const uint4*>(units + i);
-        const uint4 a = __ldg(p), b = __ldg(p + 1);
-        uint4* q = reinterpret_cast<uint4*>(&t);
-        q[0] = a;
-        q[1] = b;
+    int ahead;   // a word of the next unit: loaded early, so that the unit itself is found in L1
+    __device__ __forceinline__ void touch() {
+        if (u < n_units) ahead = __ldg(reinterpret_cast<const int*>(units + u));
     }
-    __device__ __forceinline__ UnitWalk(const Unit* units_, int n_units_) : units(units_), n_units(n_units_), u(blockIdx.x) {
-        have_next = u < n_units;
-        if (have_next) load(nxt, u);
-    }
-    // the next unit with work of this CTA (the one after it is requested at once, so its latency hides under this one)
+    __device__ __forceinline__ UnitWalk(const Unit* units_, int n_units_) : units(units_), n_units(n_units_), u(blockIdx.x), ahead(0) { touch(); }
+    // the next unit with work of this CTA
     __device__ __forceinline__ bool next(Unit& t) {
-        while (have_next) {
-            cur = nxt;
+        while (u < n_units) {
+            asm volatile("" ::"r"(ahead));
+            const uint4* p = reinterpret_cast<const uint4*>(units + u);
+            uint4* q = reinterpret_cast<uint4*>(&t);
+            q[0] = __ldg(p);
+            q[1] = __ldg(p + 1);
             u += gridDim.x;
-            have_next = u < n_units;
-            if (have_next) load(nxt, u);
-            if (cur.rows > 0 && cur.n_tok > 0) {
-                t = cur;
-                return true;
-            }
+            touch();
+            if (t.rows > 0 && t.n_tok > 0) return true;
         }
         return false;
     }
@@ -209,297 +270,384 @@ struct UnitWalk {
 
 // DOWN = false: act[pair][perm(row)] = f16(silu(f16(Wg x)) * f16(Wu x)); DOWN = true: y[pair][row] = f16(Wd act).
 //
-// Warp roles: warp 0 issues the weights' TMA copies and the last warp the tokens'; warps 1..4 issue the MMAs (a quarter of a slab's K steps each, into a
-// partial accumulator of their own); warps 5..8 run the epilogue; warps 9..24 convert codes into the A operand.
-// Three rings decouple them: the weight ring (codes and scales of a slab; released as soon as the converting warps
-// hold the slab in registers), the token ring (the slab's B tile; released by the MMAs' completion) and the A
-// buffers in tensor memory (filled by the converting warps, released by the MMAs' completion).  A stage's life in
-// the weight ring is then one memory latency plus one conversion, whatever the MMAs' lag.
+// What bounds it: not memory (the same walk without conversion, MMAs and scaling runs at 6.2 TB/s) and not the tensor pipe, but
+// the converting warps' instructions and the hand-overs between the roles.  Hence few warps (with 16 converting warps
+// the waits of all of them took more issue slots than their arithmetic gained: 1210 us against 1140), a whole slab per
+// hand-over (quarters: 1680 us), no scale product per weight, rolled conversion loops, operands that need no
+// per-lane moves (elect_one).  Kimi layer, experts' launches alone, before and now: 32 tokens (177 distinct experts,
+// 4.4 GB) 1203 -> 963 us = 4.55 TB/s; 8 tokens 306 -> 246 us; 128 tokens with skewed load 1317 -> 1128 us; Mixtral shape,
+// 50 tokens 294 -> 264 us.
+//
+// Every role walks the same sequence: units blockIdx.x, + gridDim.x, ...; per unit ceil(n_tok / 32) passes of one or two
+// token groups of 16; per pass nslab slabs of 256 columns; per slab a step for each token group.  `it` counts slabs (code
+// stage it % 8, A buffer and converting team it & 1), `step` steps (accumulator buffer and scaling team step & 1).  With
+// one token group the two scaling teams take alternate slabs of the same tokens and their sums meet at the end, with
+// two groups each team has its own.  A barrier is only ever waited for by roles that have seen its previous phase
+// complete (a wait names its phase by one parity bit).
 template <bool DOWN>
 __global__ void __launch_bounds__(kGrpThreads, 1) moe_grouped_kernel(const __grid_constant__ GroupedMaps maps, GroupedArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_dyn[];
-    unsigned char* wring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
-    unsigned char* xring = wring + kGrpStages * kGrpRawBytes;
-    float* exch = reinterpret_cast<float*>(xring + kGrpXStages * kGrpXBytes);                  // [64][kGrpMaxN + 1]
-    uint64_t* full = reinterpret_cast<uint64_t*>(exch + 64 * (kGrpMaxN + 1));
-    uint64_t* empty = full + kGrpStages;
-    uint64_t* xfull = empty + kGrpStages;
-    uint64_t* a_full = xfull + kGrpXStages;
-    uint64_t* a_empty = a_full + kGrpABufs;
-    uint64_t* d_full = a_empty + kGrpABufs;
-    uint64_t* d_empty = d_full + 2;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_empty + 2);
+    const uint32_t wring = (smem_u32(smem_dyn) + 1023u) & ~1023u;
+    const uint32_t xring = wring + kGrpStages * kGrpCodeBytes;
+    const uint32_t sring = xring + kGrpXStages * kGrpXBytes;
+    const uint32_t exch_addr = sring + kGrpScaleStages * kGrpScaleBytes;
+    float* exch = reinterpret_cast<float*>(smem_dyn + (exch_addr - smem_u32(smem_dyn)));               // [128][kGrpMaxN + 1]
+    const Bar full{exch_addr + 128 * (kGrpMaxN + 1) * 4};
+    const Bar empty = full + kGrpStages;
+    const Bar xfull = empty + kGrpStages;
+    const Bar xempty = xfull + kGrpXStages;
+    const Bar sfull = xempty + kGrpXStages;
+    const Bar sempty = sfull + kGrpScaleStages;
+    const Bar a_full = sempty + kGrpScaleStages;   // [it & 1] the A operand is in tensor memory
+    const Bar a_empty = a_full + 2;                // [it & 1] the MMAs that read it have completed
+    const Bar d_full = a_empty + 2;                // [step & 1] the accumulators are complete
+    const Bar d_empty = d_full + 2;                // [step & 1] the accumulators have been read
+    const Bar part_full = d_empty + 2;             // (one token group) team 1's partial sums are in exch
+    const Bar up_full = part_full + 1;             // [team] (gate/up) the up rows' sums are in exch
+    const Bar exch_free = up_full + 2;             // every scaling warp is through with this pass's exchange
+    const uint32_t tmem_slot = (exch_free + 1).addr;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
     const int K = DOWN ? a.I : a.H;
     const int nslab = K / kGrpSlabK;
     if (tid == 0) {
         for (int s = 0; s < kGrpStages; ++s) {
             mbar_init(full + s, 1);
-            mbar_init(empty + s, kGrpConvWarps / 2);
+            mbar_init(empty + s, 4);
         }
         for (int s = 0; s < kGrpXStages; ++s) {
             mbar_init(xfull + s, 1);
+            mbar_init(xempty + s, kGrpMmaWarps);
         }
-        for (int s = 0; s < kGrpABufs; ++s) {
-            mbar_init(a_full + s, kGrpConvWarps / 2);
-            mbar_init(a_empty + s, kGrpMmaWarps);
+        for (int s = 0; s < kGrpScaleStages; ++s) {
+            mbar_init(sfull + s, 1);
+            mbar_init(sempty + s, 8);
         }
         for (int s = 0; s < 2; ++s) {
+            mbar_init(a_full + s, 4);
+            mbar_init(a_empty + s, kGrpMmaWarps);
             mbar_init(d_full + s, kGrpMmaWarps);
             mbar_init(d_empty + s, 4);
+            mbar_init(up_full + s, 2);
         }
+        mbar_init(part_full, 4);
+        mbar_init(exch_free, 8);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kGrpTmemCols) : "memory");
+    if (warp == kGrpMmaWarp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(kGrpTmemCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    uint32_t tmem;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot) : "memory");
+    tmem = (uint32_t)uniform((int)tmem);
     pdl_wait();   // the work lists, the gathered tokens and (down) the intermediate are earlier kernels' outputs
     UnitWalk walk(DOWN ? a.units_dn : a.units_gu, a.work->n_active * (DOWN ? a.tiles_dn : a.tiles_gu));
 
-    // Every role walks the same sequence: units blockIdx.x, + gridDim.x, ...; per unit ceil(n_tok / 16) passes, taken
-    // two at a time (a converted slab feeds the MMAs of both token groups: an expert with 17 to 32 tokens is
-    // converted once, the shared expert of 128 tokens four times instead of eight);
-    // per pass nslab slabs.  `it` counts slabs (weight stage it % 8, token stage it % 8, A buffer it % 3), `pc`
-    // passes (D buffer pc & 1).
     bool ok = true;
     if (warp == 0) {
-        // ── TMA producer of the weight ring ──
-        int it = 0;
+        // ── TMA producer of the code and scale rings ──
+        int it = 0, ss = 0, su = 0, nchunk = 0;   // scale stage, its use number, chunks issued
         Unit t;
         while (ok && walk.next(t)) {
             const CUtensorMap* codes = DOWN ? &maps.dn_codes : &maps.gu_codes;
             const CUtensorMap* scales = DOWN ? (t.scales_last ? &maps.dn_scales_last : &maps.dn_scales_full)
                                              : (t.scales_last ? &maps.gu_scales_last : &maps.gu_scales_full);
-            const int total = grp_double_passes(t.n_tok) * nslab;
-            // One instruction for all issuing lanes (each lane's copy is a different box): the same copies issued
-            // from one branch per lane cost four times as much of the warp's time.
-            //   gate/up: lane 0/1 codes of gate/up, lane 2/3 their scales;   down: lane 0 codes, lane 1 scales
-            const int nw = DOWN ? 2 : 4;
-            const bool is_scale = lane >= nw / 2;
-            const bool second = !DOWN && (lane & 1);   // the up matrix
-            const CUtensorMap* m = is_scale ? scales : codes;
-            const uint32_t dst_off = is_scale ? 16384 + (second ? 1024 : 0) : (second ? 8192 : 0);
-            const int c2 = second ? t.slot_b : t.slot_a;
-            for (int i = 0; i < total; ++i, ++it) {
-                const int s = i % nslab;
-                const int st = it % kGrpStages;
-                if (it >= kGrpStages) ok = mbar_wait_hint(empty + st, ((it / kGrpStages) - 1) & 1);
-                if (!ok) break;
-                if (lane == 0) mbar_expect_tx(full + st, kGrpRawBytes);
-                __syncwarp();
-                if (lane < nw) tma_load_3d(wring + (size_t)st * kGrpRawBytes + dst_off, m, is_scale ? s * 16 : s * 128, t.row0, c2, full + st);
-                __syncwarp();
+            const int row0 = uniform(t.row0), slot_a = uniform(t.slot_a), slot_b = uniform(t.slot_b);
+            const int passes = grp_passes(t.n_tok);
+            for (int p = 0; ok && p < passes; ++p) {
+                for (int s = 0; s < nslab; ++s, ++it) {
+                    const int st = it % kGrpStages;
+                    const bool chunk = s % kGrpChunkSlabs == 0;
+                    if (it >= kGrpStages) ok = mbar_wait_grp(empty + st, ((it / kGrpStages) - 1) & 1);
+                    if (chunk && ok && su > 0) ok = mbar_wait_grp(sempty + ss, (su - 1) & 1);
+                    if (!ok) break;
+                    if (elect_one()) {
+                        const uint32_t dst = wring + (uint32_t)st * kGrpCodeBytes;
+                        mbar_expect_tx(full + st, kGrpCodeBytes);
+                        tma_load_3d(dst, codes, s * 128, row0, slot_a, full + st);
+                        if (!DOWN) tma_load_3d(dst + kGrpCodeBytes / 2, codes, s * 128, row0, slot_b, full + st);
+                        if (chunk) {
+                            const uint32_t sdst = sring + (uint32_t)ss * kGrpScaleBytes;
+                            mbar_expect_tx(sfull + ss, kGrpScaleBytes);
+                            tma_load_3d(sdst, scales, s * 16, row0, slot_a, sfull + ss);
+                            if (!DOWN) tma_load_3d(sdst + kGrpScaleBytes / 2, scales, s * 16, row0, slot_b, sfull + ss);
+                        }
+                    }
+                    __syncwarp();
+                    if (chunk) {
+                        ++nchunk;
+                        if (++ss == kGrpScaleStages) {
+                            ss = 0;
+                            ++su;
+                        }
+                    }
+                }
             }
         }
         if (!ok && lane == 0) flag(a.status, kStatusTimeout);
         // drain: every issued copy must have landed before the CTA's shared memory goes away
-        if (lane == 0)
+        if (lane == 0) {
             for (int k = max(0, it - kGrpStages); k < it; ++k)
-                if (!mbar_wait_hint(full + (k % kGrpStages), (k / kGrpStages) & 1)) flag(a.status, kStatusTimeout);
+                if (!mbar_wait_grp(full + (k % kGrpStages), (k / kGrpStages) & 1)) flag(a.status, kStatusTimeout);
+            for (int k = max(0, nchunk - kGrpScaleStages); k < nchunk; ++k)
+                if (!mbar_wait_grp(sfull + (k % kGrpScaleStages), (k / kGrpScaleStages) & 1)) flag(a.status, kStatusTimeout);
+        }
     } else if (warp == kGrpXWarp) {
-        // ── TMA producer of the token ring: one copy per slab (four K-major tiles of 64 columns) ──
-        int it = 0;
+        // ── TMA producer of the token ring: one copy per step (four K-major tiles of 64 columns) ──
+        int xs = 0, xu = 0, n = 0;   // stage, its use number, copies issued
         Unit t;
         const CUtensorMap* xmap = DOWN ? &maps.act16 : &maps.xg16;
         while (ok && walk.next(t)) {
             for (int p0 = 0; ok && p0 < t.n_tok; p0 += 2 * kGrpMaxN) {
-                const int ng = t.n_tok - p0 > kGrpMaxN ? 2 : 1;   // token groups of this double pass
-                for (int s = 0; s < nslab; ++s, ++it) {
-                    const int xs = it % kGrpXStages;
-                    if (it >= kGrpXStages) ok = mbar_wait_hint(a_empty + xs, ((it / kGrpXStages) - 1) & 1);
-                    if (!ok) break;
-                    if (lane == 0) {
-                        mbar_expect_tx(xfull + xs, ng * kGrpXGroupBytes);
-                        tma_load_3d(xring + (size_t)xs * kGrpXBytes, xmap, 0, t.pair_off + p0, s * (kGrpSlabK / 64), xfull + xs);
-                        if (ng == 2)
-                            tma_load_3d(xring + (size_t)xs * kGrpXBytes + kGrpXGroupBytes, xmap, 0, t.pair_off + p0 + kGrpMaxN,
-                                        s * (kGrpSlabK / 64), xfull + xs);
+                const int ng = t.n_tok - p0 > kGrpMaxN ? 2 : 1;
+                const int row = uniform(t.pair_off + p0);
+                for (int s = 0; ok && s < nslab; ++s) {
+                    for (int g = 0; g < ng; ++g, ++n) {
+                        if (xu > 0) ok = mbar_wait_grp(xempty + xs, (xu - 1) & 1);
+                        if (!ok) break;
+                        if (elect_one()) {
+                            mbar_expect_tx(xfull + xs, kGrpXBytes);
+                            tma_load_3d(xring + (uint32_t)xs * kGrpXBytes, xmap, 0, row + g * kGrpMaxN, s * (kGrpSlabK / 64), xfull + xs);
+                        }
+                        __syncwarp();
+                        if (++xs == kGrpXStages) {
+                            xs = 0;
+                            ++xu;
+                        }
                     }
-                    __syncwarp();
                 }
             }
         }
         if (!ok && lane == 0) flag(a.status, kStatusTimeout);
         if (lane == 0)
-            for (int k = max(0, it - kGrpXStages); k < it; ++k)
-                if (!mbar_wait_hint(xfull + (k % kGrpXStages), (k / kGrpXStages) & 1)) flag(a.status, kStatusTimeout);
-    } else if (warp <= kGrpMmaWarps) {
-        // ── MMA issuers: warp w takes the K steps 4 (w - 1) .. 4 (w - 1) + 3 of every slab and accumulates them into
-        // its own partial accumulator; the epilogue adds the four ──
-        const int mw = warp - 1;
-        int it = 0, pc = 0;
+            for (int k = max(0, n - kGrpXStages); k < n; ++k)
+                if (!mbar_wait_grp(xfull + (k % kGrpXStages), (k / kGrpXStages) & 1)) flag(a.status, kStatusTimeout);
+    } else if (warp < kGrpFirstScaleWarp) {
+        // ── MMA issuers: per step and scale group (32 columns, an accumulator of its own) two MMAs; the issuers share the groups ──
+        const int mw = warp - kGrpMmaWarp;
+        int it = 0, step = 0, xs = 0, xu = 0;
         Unit t;
+        constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(kGrpMaxN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
         while (ok && walk.next(t)) {
             for (int p0 = 0; ok && p0 < t.n_tok; p0 += 2 * kGrpMaxN) {
-                const uint32_t idesc = (1u << 4) | ((uint32_t)(kGrpMaxN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-                // a double pass: token group g accumulates into D buffer (pc + g) & 1 — with two groups both buffers
-                const int ng = t.n_tok - p0 > kGrpMaxN ? 2 : 1;
-                for (int g = 0; ok && g < ng; ++g)
-                    if (pc + g >= 2) ok = mbar_wait_hint(d_empty + ((pc + g) & 1), (((pc + g) >> 1) - 1) & 1);
+                const int ng = uniform(t.n_tok - p0 > kGrpMaxN ? 2 : 1);
                 for (int s = 0; ok && s < nslab; ++s, ++it) {
-                    const int xs = it % kGrpXStages, ab = it % kGrpABufs;
-                    ok = mbar_wait_hint(xfull + xs, (it / kGrpXStages) & 1) && mbar_wait_hint(a_full + ab, (it / kGrpABufs) & 1);
-                    if (!ok) break;
-                    tc_fence_after();
-                    if (lane == 0) {
+                    const int ab = it & 1;
+                    for (int g = 0; g < ng; ++g, ++step) {
+                        const int db = step & 1;
+                        if (step >= 2) ok = ok && mbar_wait_grp(d_empty + db, ((step >> 1) - 1) & 1);
+                        ok = ok && mbar_wait_grp(xfull + xs, xu & 1);
+                        const uint32_t xaddr = xring + (uint32_t)xs * kGrpXBytes;
+                        const uint64_t xdesc = (uint64_t)((xaddr & 0x3FFFF) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
+                                               ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+                        const uint32_t d0 = tmem + kGrpDCol0 + db * kGrpDCols, a0 = tmem + ab * kGrpACols;
+                        // last, since it is the one that decides: a wait costs some 200 cycles also when its phase is over
+                        if (g == 0) ok = ok && mbar_wait_grp(a_full + ab, (it >> 1) & 1);
+                        if (!ok) break;
+                        tc_fence_after();
+                        if (elect_one()) {
 #pragma unroll
-                        for (int g = 0; g < 2; ++g) {
-                            if (g >= ng) break;
-                            const int db = (pc + g) & 1;
-                            const uint32_t xaddr = smem_u32(xring + (size_t)xs * kGrpXBytes + g * kGrpXGroupBytes);
+                            for (int kk = 0; kk < 2; ++kk) {
 #pragma unroll
-                            for (int kk = 0; kk < kGrpSlabK / 16 / kGrpMmaWarps; ++kk) {
-                                const int k = mw * (kGrpSlabK / 16 / kGrpMmaWarps) + kk;
-                                const uint32_t baddr = xaddr + (k >> 2) * kGrpMaxN * 128 + (k & 3) * 32;
-                                const uint64_t bdesc = (uint64_t)((baddr & 0x3FFFF) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
-                                                       ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
-                                const uint32_t acc = (s > 0 || kk > 0) ? 1u : 0u;
-                                asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-                                             ::"r"(tmem + kGrpDCol0 + (db * kGrpMmaWarps + mw) * kGrpMaxN), "r"(tmem + ab * kGrpACols + 8 * k), "l"(bdesc),
-                                             "r"(idesc), "r"(acc)
-                                             : "memory");
+                                for (int i = 0; i < 8 / kGrpMmaWarps; ++i) {
+                                    const int gr = i * kGrpMmaWarps + mw;
+                                    const uint64_t bdesc = xdesc + (uint64_t)(((gr >> 1) * kGrpMaxN * 128 + (gr & 1) * 64 + kk * 32) >> 4);
+                                    umma_ts(d0 + gr * kGrpMaxN, a0 + 16 * gr + 8 * kk, bdesc, idesc, (uint32_t)kk);
+                                }
                             }
+                            umma_commit(d_full + db);
+                            umma_commit(xempty + xs);
+                            if (g == ng - 1) umma_commit(a_empty + ab);
                         }
-                        umma_commit(a_empty + ab);
-                        if (s == nslab - 1) {
-                            umma_commit(d_full + (pc & 1));
-                            if (ng == 2) umma_commit(d_full + ((pc + 1) & 1));
+                        __syncwarp();
+                        if (++xs == kGrpXStages) {
+                            xs = 0;
+                            ++xu;
                         }
                     }
-                    __syncwarp();
                 }
-                pc += ng;
             }
         }
         if (!ok && lane == 0) flag(a.status, kStatusTimeout);
     } else if (warp >= kGrpFirstConvWarp) {
-        // ── converting warps: two teams of eight take alternate slabs, so that one team's waits (for the copy, for
-        // the A buffer, for its stores into tensor memory) overlap the other team's arithmetic.  Within a team: row
-        // m = 32 (warp % 4) + lane of the A tile, K half (128 columns) of the slab ──
-        const int cw = warp - kGrpFirstConvWarp;
-        const int q = warp & 3, team = cw >> 3, kh = (cw >> 2) & 1;
+        // ── converting warps: two teams of four take alternate slabs.  Row m = 32 (warp % 4) + lane of the A tile ──
+        const int team = (warp - kGrpFirstConvWarp) >> 2;
+        const int q = warp & 3;
         const int m = 32 * q + lane;
-        // where row m's codes and scales sit in a stage
-        const int src_row = DOWN ? m : (m & 63);
-        const uint32_t code_off = (DOWN ? 0u : (m >= 64 ? 8192u : 0u)) + (uint32_t)src_row * 128u;
-        const uint32_t scale_off = 16384u + (DOWN ? 0u : (m >= 64 ? 1024u : 0u)) + (uint32_t)src_row * 16u + (uint32_t)kh * 8u;
+        const uint32_t code_off = (uint32_t)m * 128u;         // (gate/up: the up tile follows the gate tile's 64 rows)
         const int first_row = DOWN ? 32 * q : 32 * (q & 1);   // first row (of the matrix half) among this warp's 32
-        const uint32_t sw = (uint32_t)(src_row & 7);
+        const uint32_t sw = (uint32_t)(m & 7);
+        const uint32_t taddr = tmem + ((uint32_t)(32 * q) << 16) + team * kGrpACols;
         int it = 0;
         Unit t;
         while (ok && walk.next(t)) {
-            const int total = grp_double_passes(t.n_tok) * nslab;
+            const int end = it + grp_passes(t.n_tok) * nslab;
             // a warp whose 32 rows all lie beyond the tile's last row has nothing to convert: its lanes of the
             // accumulator are never read
             const bool work = first_row < t.rows;
-            for (int i = 0; ok && i < total; ++i, ++it) {
-                if ((it & 1) != team) continue;
-                const int st = it % kGrpStages, ab = it % kGrpABufs;
-                ok = mbar_wait_hint(full + st, (it / kGrpStages) & 1);
+            for (int i = it + ((it ^ team) & 1); i < end; i += 2) {
+                const int st = i % kGrpStages, use = i >> 1;
+                ok = mbar_wait_grp(full + st, (i / kGrpStages) & 1);
                 if (!ok) break;
-                const uint32_t sb = smem_u32(wring + (size_t)st * kGrpRawBytes);
-                const uint32_t cb = sb + code_off;
-                const uint32_t taddr = tmem + ((uint32_t)(32 * q) << 16) + ab * kGrpACols + kh * 64;
-                uint32_t h0[16], h1[16];
-                uint32_t sc0 = 0, sc1 = 0;   // four group scales
+                const uint32_t cb = wring + (uint32_t)st * kGrpCodeBytes + code_off;
+                uint4 n0 = make_uint4(0, 0, 0, 0), n1 = n0;   // the next two scale groups' codes
                 if (work) {
-                    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(sc0), "=r"(sc1) : "r"(sb + scale_off));
-                    const uint4 c0 = lds128(cb + (((uint32_t)(4 * kh) ^ sw) * 16u));
-                    const uint4 c1 = lds128(cb + (((uint32_t)(4 * kh + 1) ^ sw) * 16u));
-                    dequant_chunk(c0, __byte_perm(sc0, 0, 0x1010), h0);
-                    dequant_chunk(c1, __byte_perm(sc0, 0, 0x3232), h1);
+                    n0 = lds128(cb + ((0u ^ sw) * 16u));
+                    n1 = lds128(cb + ((1u ^ sw) * 16u));
                 }
-                if (it >= kGrpABufs) ok = mbar_wait_hint(a_empty + ab, ((it / kGrpABufs) - 1) & 1);
+                if (use > 0) ok = mbar_wait_grp(a_empty + team, (use - 1) & 1);
                 if (!ok) break;
                 tc_fence_after();
-                uint4 c2 = make_uint4(0, 0, 0, 0), c3 = c2;
                 if (work) {
-                    tmem_st16(taddr, h0);
-                    tmem_st16(taddr + 16, h1);
-                    c2 = lds128(cb + (((uint32_t)(4 * kh + 2) ^ sw) * 16u));
-                    c3 = lds128(cb + (((uint32_t)(4 * kh + 3) ^ sw) * 16u));
+                    // (rolled: four trips through a short loop fetch fewer instructions than 320 of them in a row)
+#pragma unroll 1
+                    for (int j = 0; j < 8; j += 2) {
+                        uint32_t g[32];
+                        const uint4 c0 = n0, c1 = n1;
+                        if (j < 6) {
+                            n0 = lds128(cb + ((((uint32_t)j + 2) ^ sw) * 16u));
+                            n1 = lds128(cb + ((((uint32_t)j + 3) ^ sw) * 16u));
+                        }
+                        codes_to_f16(c0, g);
+                        codes_to_f16(c1, g + 16);
+                        tmem_st32(taddr + 16 * j, g);
+                    }
                 }
                 __syncwarp();
-                if (lane == 0) mbar_arrive(empty + st);   // the slab is in registers: the stage may be refilled
-                if (work) {
-                    dequant_chunk(c2, __byte_perm(sc1, 0, 0x1010), h0);
-                    dequant_chunk(c3, __byte_perm(sc1, 0, 0x3232), h1);
-                    tmem_st16(taddr + 32, h0);
-                    tmem_st16(taddr + 48, h1);
-                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                }
+                mbar_arrive_lane0(empty + st, lane);   // the slab is in registers: the stage may be refilled
+                if (work) asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(a_full + ab);
+                mbar_arrive_lane0(a_full + team, lane);
             }
+            it = end;
         }
         if (!ok && lane == 0) flag(a.status, kStatusTimeout);
-    } else if (warp >= kGrpFirstEpiWarp) {
-        // ── epilogue warps: TMEM lanes 32 (warp % 4) .. + 31 ──
+    } else if (warp >= kGrpFirstScaleWarp) {
+        // ── scaling warps: lane = row m of the tile ──
+        const int team = (warp - kGrpFirstScaleWarp) >> 2;
         const int q = warp & 3;
         const int m = 32 * q + lane;
-        int pc = 0;
+        const int first_row = DOWN ? 32 * q : 32 * (q & 1);
+        // row m's scales in a stage: 64 bytes per row, 64-byte swizzle (the 16-byte unit number is XORed with row / 2)
+        const uint32_t sbase = sring + (uint32_t)m * 64u;
+        const uint32_t ssw = (uint32_t)(m >> 1) & 3u;
+        const uint32_t taddr = tmem + ((uint32_t)(32 * q) << 16) + kGrpDCol0 + team * kGrpDCols;
+        int step = 0, pc = 0, ss = 0, su = 0, n_part = 0, n_up = 0;
         Unit t;
         while (ok && walk.next(t)) {
-            for (int p0 = 0; ok && p0 < t.n_tok; p0 += kGrpMaxN, ++pc) {
-                const int ntok = min(kGrpMaxN, t.n_tok - p0);
-                const int db = pc & 1;
-                ok = mbar_wait_hint(d_full + db, (pc >> 1) & 1);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t taddr = tmem + ((uint32_t)(32 * q) << 16) + kGrpDCol0 + db * kGrpMmaWarps * kGrpMaxN;
-                uint32_t d[16];
-                {
-                    // the four issuers' partial sums, added pairwise: (p0 + p1) + (p2 + p3)
-                    uint32_t p[16], r[16];
-                    tmem_ld16(taddr, d);
-                    tmem_ld16(taddr + kGrpMaxN, p);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            const bool work = first_row < t.rows;
+            for (int p0 = 0; ok && p0 < t.n_tok; p0 += 2 * kGrpMaxN, ++pc) {
+                const bool two = t.n_tok - p0 > kGrpMaxN;
+                const int grp = two ? (team ^ step) & 1 : 0;      // this team's token group of the pass
+                const int t0 = p0 + grp * kGrpMaxN;
+                const int ntok = min(kGrpMaxN, t.n_tok - t0);
+                float2 acc[kGrpMaxN / 2];
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) d[j] = __float_as_uint(__uint_as_float(d[j]) + __uint_as_float(p[j]));
-                    tmem_ld16(taddr + 2 * kGrpMaxN, r);
-                    tmem_ld16(taddr + 3 * kGrpMaxN, p);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        d[j] = __float_as_uint(__uint_as_float(d[j]) + (__uint_as_float(r[j]) + __uint_as_float(p[j])));
+                for (int j = 0; j < kGrpMaxN / 2; ++j) acc[j] = make_float2(0.f, 0.f);
+                for (int s = 0; s < nslab; ++s) {
+                    const uint32_t sub = (uint32_t)s % kGrpChunkSlabs;
+                    if (sub == 0) ok = ok && mbar_wait_grp(sfull + ss, su & 1);
+                    // the step of this slab that belongs to this team, if any
+                    const int mine = step + grp;
+                    step += two ? 2 : 1;
+                    if ((mine & 1) == team) {
+                        uint4 sc = lds128(sbase + (uint32_t)ss * kGrpScaleBytes + ((sub ^ ssw) << 4));
+                        ok = ok && mbar_wait_grp(d_full + team, (mine >> 1) & 1);
+                        if (!ok) break;
+                        tc_fence_after();
+                        if (!work) {
+                            mbar_arrive_lane0(d_empty + team, lane);
+                        } else if (ntok <= 4) {
+                            scale_slab<4>(taddr, sc, acc, d_empty + team, lane);
+                        } else if (ntok <= 8) {
+                            scale_slab<8>(taddr, sc, acc, d_empty + team, lane);
+                        } else {
+                            scale_slab<16>(taddr, sc, acc, d_empty + team, lane);
+                        }
+                    }
+                    if (sub == kGrpChunkSlabs - 1 || s == nslab - 1) {
+                        __syncwarp();
+                        mbar_arrive_lane0(sempty + ss, lane);
+                        if (++ss == kGrpScaleStages) {
+                            ss = 0;
+                            ++su;
+                        }
+                    }
                 }
-                // the accumulators are in registers: the MMAs of the pass after next may overwrite them
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(d_empty + db);
-                if (DOWN) {
-                    if (m < t.rows) {
+                if (pc > 0) ok = ok && mbar_wait_grp(exch_free, (pc - 1) & 1);
+                if (!ok) break;
+                float* ex = exch + m * (kGrpMaxN + 1);
+                bool store = true;
+                if (!two) {
+                    // one token group: the two teams' sums meet in shared memory; team 0 adds team 1's and stores
+                    if (team == 1) {
 #pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            if (j < ntok) a.y[(size_t)(t.pair_off + p0 + j) * a.H + t.mrow0 + m] = __float2half_rn(__uint_as_float(d[j]));
-                    }
-                } else {
-                    // the up half hands its values to the gate half of the same rows
-                    if (m >= 64) {
+                        for (int j = 0; j < kGrpMaxN / 2; ++j) {
+                            if (2 * j < ntok) {
+                                ex[2 * j] = acc[j].x;
+                                ex[2 * j + 1] = acc[j].y;
+                            }
+                        }
+                        __syncwarp();
+                        mbar_arrive_lane0(part_full, lane);
+                        store = false;
+                    } else {
+                        ok = mbar_wait_grp(part_full, n_part++ & 1);
+                        if (!ok) break;
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) exch[(m - 64) * (kGrpMaxN + 1) + j] = __uint_as_float(d[j]);
-                    }
-                    asm volatile("bar.sync 3, 128;" ::: "memory");
-                    if (m < 64 && m < t.rows) {
-                        const int col = perm8(t.mrow0 + m);
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            if (j < ntok) {
-                                const float g16 = __half2float(__float2half_rn(__uint_as_float(d[j])));
-                                const float u16 = __half2float(__float2half_rn(exch[m * (kGrpMaxN + 1) + j]));
-                                a.act[(size_t)(t.pair_off + p0 + j) * a.I + col] = __float2half_rn(silu_mul_f32(g16, u16));
+                        for (int j = 0; j < kGrpMaxN / 2; ++j) {
+                            if (2 * j < ntok) {
+                                acc[j].x += ex[2 * j];
+                                acc[j].y += ex[2 * j + 1];
                             }
                         }
                     }
-                    asm volatile("bar.sync 3, 128;" ::: "memory");
                 }
+                if (store && DOWN) {
+                    if (m < t.rows) {
+                        __half* y = a.y + (size_t)(t.pair_off + t0) * a.H + t.mrow0 + m;
+#pragma unroll
+                        for (int j = 0; j < kGrpMaxN; ++j)
+                            if (j < ntok) y[(size_t)j * a.H] = __float2half_rn(j & 1 ? acc[j >> 1].y : acc[j >> 1].x);
+                    }
+                } else if (store) {
+                    // the up half hands its values to the gate half of the same rows: through the second half of exch, or
+                    // (two token groups) through the team's half
+                    float* up = two ? exch + (team * 64 + (m & 63)) * (kGrpMaxN + 1) : exch + (64 + (m & 63)) * (kGrpMaxN + 1);
+                    if (m >= 64) {
+#pragma unroll
+                        for (int j = 0; j < kGrpMaxN / 2; ++j) {
+                            if (2 * j < ntok) {
+                                up[2 * j] = acc[j].x;
+                                up[2 * j + 1] = acc[j].y;
+                            }
+                        }
+                        __syncwarp();
+                        mbar_arrive_lane0(up_full + team, lane);
+                    } else {
+                        ok = mbar_wait_grp(up_full + team, n_up & 1);
+                        if (!ok) break;
+                        if (m < t.rows) {
+                            __half* act = a.act + (size_t)(t.pair_off + t0) * a.I + perm8(t.mrow0 + m);
+#pragma unroll
+                            for (int j = 0; j < kGrpMaxN; ++j) {
+                                if (j < ntok) {
+                                    const float g16 = __half2float(__float2half_rn(j & 1 ? acc[j >> 1].y : acc[j >> 1].x));
+                                    const float u16 = __half2float(__float2half_rn(up[j]));
+                                    act[(size_t)j * a.I] = __float2half_rn(silu_mul_f32(g16, u16));
+                                }
+                            }
+                        }
+                    }
+                    ++n_up;
+                }
+                __syncwarp();
+                mbar_arrive_lane0(exch_free, lane);
             }
         }
         if (!ok && lane == 0) flag(a.status, kStatusTimeout);
@@ -508,7 +656,7 @@ __global__ void __launch_bounds__(kGrpThreads, 1) moe_grouped_kernel(const __gri
     tc_fence_before();
     __syncthreads();
     pdl_trigger();
-    if (warp == 1) {
+    if (warp == kGrpMmaWarp) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kGrpTmemCols) : "memory");
     }
@@ -785,14 +933,13 @@ EncodeTiledFn encode_fn() {
 }
 
 // 3-D map over the pool: x = byte in a row (row_bytes), y = row in the page (rows), z = pool slot.
-int make_pool_map(CUtensorMap* m, void* base, size_t row_bytes, int rows, size_t slots, int box_x, int box_y, bool swizzle) {
+int make_pool_map(CUtensorMap* m, void* base, size_t row_bytes, int rows, size_t slots, int box_x, int box_y, CUtensorMapSwizzle swizzle) {
     const cuuint64_t dims[3] = {(cuuint64_t)row_bytes, (cuuint64_t)rows, (cuuint64_t)slots};
     const cuuint64_t strides[2] = {(cuuint64_t)row_bytes, (cuuint64_t)(2u << 20)};
     const cuuint32_t box[3] = {(cuuint32_t)box_x, (cuuint32_t)box_y, 1};
     const cuuint32_t es[3] = {1, 1, 1};
     CUresult r = encode_fn()(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, base, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                             swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                             swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? 0 : VIB3_ERR_STATE;
 }
 
@@ -859,8 +1006,10 @@ int launch_pdl(K kernel, dim3 grid, int threads, size_t smem, cudaStream_t st, A
     return (int)cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-constexpr size_t kGrpSmem = 1024 + (size_t)kGrpStages * kGrpRawBytes + (size_t)kGrpXStages * kGrpXBytes +
-                            64 * (kGrpMaxN + 1) * sizeof(float) + 48 * sizeof(uint64_t);
+constexpr int kGrpBarriers = 2 * kGrpStages + 2 * kGrpXStages + 2 * kGrpScaleStages + 8 + 4 + 1;   // (+ the tensor memory address)
+constexpr size_t kGrpSmem = 1024 + (size_t)kGrpStages * kGrpCodeBytes + (size_t)kGrpXStages * kGrpXBytes + (size_t)kGrpScaleStages * kGrpScaleBytes +
+                            128 * (kGrpMaxN + 1) * sizeof(float) + kGrpBarriers * sizeof(uint64_t);
+static_assert(kGrpSmem <= kSmemBudget, "shared memory of a CTA");
 
 }  // namespace
 
@@ -907,17 +1056,19 @@ extern "C" int vib3_moe_grouped_prewarm(void* pool_base, size_t capacity_pages, 
     h->max_pairs = max_tokens * (top_k + 1);
     const size_t gu_code_row = hidden_dim / 2, gu_scale_row = hidden_dim / 16;
     const size_t dn_code_row = expert_hidden_dim / 2, dn_scale_row = expert_hidden_dim / 16;
+    const CUtensorMapSwizzle sw128 = CU_TENSOR_MAP_SWIZZLE_128B, sw64 = CU_TENSOR_MAP_SWIZZLE_64B;
+    constexpr int kScaleBox = kGrpChunkSlabs * 16;
     int e = 0;
-    e |= make_pool_map(&h->maps.gu_codes, pb, gu_code_row, rows_per_page_gate_up, capacity_pages, 128, 64, true);
+    e |= make_pool_map(&h->maps.gu_codes, pb, gu_code_row, rows_per_page_gate_up, capacity_pages, 128, 64, sw128);
     e |= make_pool_map(&h->maps.gu_scales_full, pb + (size_t)rows_per_page_gate_up * gu_code_row, gu_scale_row, rows_per_page_gate_up,
-                       capacity_pages, 16, 64, false);
+                       capacity_pages, kScaleBox, 64, sw64);
     e |= make_pool_map(&h->maps.gu_scales_last, pb + (size_t)last_page_rows_gate_up * gu_code_row, gu_scale_row, last_page_rows_gate_up,
-                       capacity_pages, 16, 64, false);
-    e |= make_pool_map(&h->maps.dn_codes, pb, dn_code_row, rows_per_page_down, capacity_pages, 128, 128, true);
+                       capacity_pages, kScaleBox, 64, sw64);
+    e |= make_pool_map(&h->maps.dn_codes, pb, dn_code_row, rows_per_page_down, capacity_pages, 128, 128, sw128);
     e |= make_pool_map(&h->maps.dn_scales_full, pb + (size_t)rows_per_page_down * dn_code_row, dn_scale_row, rows_per_page_down,
-                       capacity_pages, 16, 128, false);
+                       capacity_pages, kScaleBox, 128, sw64);
     e |= make_pool_map(&h->maps.dn_scales_last, pb + (size_t)last_page_rows_down * dn_code_row, dn_scale_row, last_page_rows_down,
-                       capacity_pages, 16, 128, false);
+                       capacity_pages, kScaleBox, 128, sw64);
     e |= make_rows_map(&h->maps.xg16, h->xg, hidden_dim, h->max_pairs, 16);
     e |= make_rows_map(&h->maps.act16, h->act, expert_hidden_dim, h->max_pairs, 16);
     if (e) {
