@@ -214,3 +214,26 @@ def test_exact_order_bound_under_stress(cuda_dev, oracle, case):
             assert np.allclose(ws_n[t], ow, rtol=2e-4), t
     assert bad == 0, f"{bad} of {T} tokens selected other experts than the CPU router ({case})"
     assert int(wk[:, 1].sum().item()) > 0 or case == "offset"   # the recomputation path was taken at least once
+
+
+@pytest.mark.parametrize("E,H,ntok,xdt,wdt", [
+    (5, 264, 9, torch.bfloat16, torch.float32), (3, 128, 12, torch.float16, torch.float16), (384, 1024, 13, torch.float32, torch.float32),
+    (7, 2056, 48, torch.bfloat16, torch.float16), (64, 520, 49, torch.float16, torch.float32), (16, 7168, 128, torch.bfloat16, torch.float32)])
+def test_batched_logits_equal_single_token_logits(cuda_dev, E, H, ntok, xdt, wdt):
+    """Token counts around the widths of the batched kernel, expert counts that leave rows of a CTA empty, row lengths that
+    leave lanes without an item: every logit is the single-token launch's bit for bit."""
+    from vic_b200 import kernels
+    g = torch.Generator(device=cuda_dev).manual_seed(E * H + ntok)
+    W = (0.05 * torch.randn(E, H, generator=g, device=cuda_dev)).to(wdt)
+    xs = torch.randn(ntok, H, generator=g, device=cuda_dev).to(xdt)
+    k = min(3, E)
+    def buffers(n):
+        return (torch.zeros(n, 3 * E, device=cuda_dev), torch.zeros(n, 16, dtype=torch.int16, device=cuda_dev),
+                torch.zeros(n, 16, device=cuda_dev), torch.zeros(n, 4, dtype=torch.int32, device=cuda_dev))
+    sc, ids, wt, ws = buffers(ntok)
+    kernels.router_topk_batch(xs, W, sc, None, None, ids, wt, k, 1, 2.5, True, 0, ws)
+    for t in range(ntok):
+        s1, i1, w1, ws1 = buffers(1)
+        kernels.router_topk_batch(xs[t:t + 1], W, s1, None, None, i1, w1, k, 1, 2.5, True, 0, ws1)
+        torch.cuda.synchronize()
+        assert torch.equal(sc[t, :E], s1[0, :E]) and torch.equal(ids[t], i1[0]) and torch.equal(wt[t], w1[0]), t

@@ -33,7 +33,7 @@
 // selection scores among the best k+1 are closer than a bound on the summation-order
 // difference, the near-tied experts' logits are recomputed with one sequential multiply-then-add
 // chain per expert (the CPU order) before the final selection (router_core.cuh).  This costs about
-// 20 microseconds and happens for a few percent of tokens.
+// 26 microseconds and happens for a few percent of tokens.
 #include "pipe_common.cuh"
 #include "router_core.cuh"
 
@@ -260,17 +260,151 @@ __global__ void __launch_bounds__(kRowsThreads) router_rows_kernel(RouterArgs a,
     }
 }
 
-__global__ void __launch_bounds__(kRouterThreads) router_select_kernel(RouterArgs a) {
+// router_rows_batch_kernel: the first launch for many tokens.  The rows of the CTA lie in shared memory as above; a warp
+// forms the logits of all three rows for TB tokens at once, so that a weight read from shared memory serves TB tokens and an
+// activation, read straight from the L2 cache by the lane that needs it, serves three rows.  With one (row, token) per warp
+// the reads from shared memory bound the launch: 6 bytes per product, 129 thousand cycles at 128 tokens of the Kimi
+// shape; here it is 1 byte, and the multiply-adds (two per product: the sum, and the sum of magnitudes for the
+// near-tie bound, two at a time) come first.  The order of a logit's sum is the same (lane l owns chains 4l .. 4l + 3).
+// Whole batched router without recomputations, one (row, token) per warp -> here, bf16 tokens, Kimi shape: 16 tokens
+// 18.8 -> 16.5 us, 32: 33.2 -> 18.8, 128: 120.6 -> 53.6; 8 experts of 4096: 16 tokens 12.7 -> 10.7 us, 128: 79.4 -> 14.7.  Up to
+// 8 tokens the other kernel is the faster one (Kimi 11.5 against 14.2 us: too few warps have a token here); at 12 they tie.
+constexpr int kBatchWarps = 12;
+constexpr int kBatchThreads = kBatchWarps * 32;
+constexpr int kBatchMinTokens = 8;
+
+// acc += a b on both halves: two independent fp32 FMAs in one issue slot
+__device__ __forceinline__ void fma2(float2& acc, const float2& a, const float2& b) {
+    uint64_t c, x, y;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(c) : "f"(acc.x), "f"(acc.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(a.x), "f"(a.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "f"(b.x), "f"(b.y));
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(x), "l"(y));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(acc.x), "=f"(acc.y) : "l"(c));
+}
+
+template <int XD, int WD, int TB>
+__global__ void __launch_bounds__(kBatchThreads) router_rows_batch_kernel(RouterArgs a, int n_tokens) {
+    extern __shared__ __align__(128) unsigned char rsm[];
+    using XT = typename XItem<XD>::T;
+    const unsigned row_bytes = (unsigned)a.H * (WD == W_F32 ? 4u : 2u);
+    uint64_t* full = reinterpret_cast<uint64_t*>(rsm + kRowsPerCta * row_bytes);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int e0 = blockIdx.x * kRowsPerCta;
+    const int nrows = min(kRowsPerCta, a.E - e0);
+    if (tid == 0) {
+        if (!a.hold_dependents) pdl_trigger();
+        mbar_init(full, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        mbar_expect_tx(full, nrows * row_bytes);
+        for (int r = 0; r < nrows; ++r)
+            bulk_load(rsm + (size_t)r * row_bytes, reinterpret_cast<const unsigned char*>(a.W) + (size_t)(e0 + r) * row_bytes, row_bytes, full);
+    }
+    __syncthreads();
+    pdl_wait();   // the tokens are the predecessor's output
+    if (a.hold_dependents && tid == 0) pdl_trigger();   // (see router_rows_kernel)
+    const bool landed = mbar_wait(full, 0);
+    const int n4 = a.H >> 2;
+    for (int t0 = (blockIdx.y * kBatchWarps + warp) * TB; t0 < n_tokens; t0 += gridDim.y * kBatchWarps * TB) {
+        if (!landed) {
+            if (lane == 0 && a.counter) a.counter[(size_t)t0 * a.counter_stride + 3] = 1u;
+            continue;
+        }
+        const XT* xrow[TB];
+#pragma unroll
+        for (int t = 0; t < TB; ++t)   // (a token beyond the last repeats the last; its results are not stored)
+            xrow[t] = reinterpret_cast<const XT*>(reinterpret_cast<const unsigned char*>(a.x) + (size_t)min(t0 + t, n_tokens - 1) * a.x_stride);
+        float2 acc[kRowsPerCta][TB][2], ab[kRowsPerCta][TB];   // chains (4l, 4l + 1) and (4l + 2, 4l + 3); sums of magnitudes
+#pragma unroll
+        for (int r = 0; r < kRowsPerCta; ++r)
+#pragma unroll
+            for (int t = 0; t < TB; ++t) ab[r][t] = acc[r][t][0] = acc[r][t][1] = make_float2(0.f, 0.f);
+        // the activations of the next two steps are in flight under this one's arithmetic
+        constexpr int kAhead = 2;
+        XT xq[kAhead][TB];
+#pragma unroll
+        for (int d = 0; d < kAhead; ++d)
+#pragma unroll
+            for (int t = 0; t < TB; ++t)
+                if (lane + 32 * d < n4) xq[d][t] = xrow[t][lane + 32 * d];
+#pragma unroll 1
+        for (int i0 = lane; i0 < n4; i0 += 32 * kAhead) {
+#pragma unroll
+            for (int d = 0; d < kAhead; ++d) {
+                const int i = i0 + 32 * d;
+                if (i >= n4) break;
+                XT cur[TB];
+#pragma unroll
+                for (int t = 0; t < TB; ++t) cur[t] = xq[d][t];
+                if (i + 32 * kAhead < n4) {
+#pragma unroll
+                    for (int t = 0; t < TB; ++t) xq[d][t] = xrow[t][i + 32 * kAhead];
+                }
+                float2 xv[TB][2], xa[TB][2];
+#pragma unroll
+                for (int t = 0; t < TB; ++t) {
+                    const float4 v = x_item<XD>(reinterpret_cast<const unsigned char*>(&cur[t]), 0);
+                    xv[t][0] = make_float2(v.x, v.y);
+                    xv[t][1] = make_float2(v.z, v.w);
+                    xa[t][0] = make_float2(fabsf(v.x), fabsf(v.y));
+                    xa[t][1] = make_float2(fabsf(v.z), fabsf(v.w));
+                }
+#pragma unroll
+                for (int r = 0; r < kRowsPerCta; ++r) {
+                    if (r >= nrows) break;
+                    const unsigned char* wrow = rsm + (size_t)r * row_bytes;
+                    const float4 wv = WD == W_F32 ? reinterpret_cast<const float4*>(wrow)[i] : WItem<W_F16>::cvt(reinterpret_cast<const uint2*>(wrow)[i]);
+                    const float2 w0 = make_float2(wv.x, wv.y), w1 = make_float2(wv.z, wv.w);
+                    const float2 a0 = make_float2(fabsf(wv.x), fabsf(wv.y)), a1 = make_float2(fabsf(wv.z), fabsf(wv.w));
+#pragma unroll
+                    for (int t = 0; t < TB; ++t) {
+                        fma2(acc[r][t][0], xv[t][0], w0);
+                        fma2(acc[r][t][1], xv[t][1], w1);
+                        fma2(ab[r][t], xa[t][0], a0);
+                        fma2(ab[r][t], xa[t][1], a1);
+                    }
+                }
+            }
+        }
+        // lane r TB + t finishes the logit of row r and token t
+        float logit = 0.f, absum = 0.f;
+#pragma unroll
+        for (int r = 0; r < kRowsPerCta; ++r)
+#pragma unroll
+            for (int t = 0; t < TB; ++t) {
+                const float c[4] = {acc[r][t][0].x, acc[r][t][0].y, acc[r][t][1].x, acc[r][t][1].y};
+                const float z = __shfl_sync(0xffffffffu, chain_tree(c), 0), s = warp_total(ab[r][t].x + ab[r][t].y);
+                if (lane == r * TB + t) {
+                    logit = z;
+                    absum = s;
+                }
+            }
+        const int r = lane / TB, t = t0 + lane % TB;
+        if (r < nrows && t < n_tokens) {
+            const int e = e0 + r;
+            float* sc = a.scores + (size_t)t * a.scores_stride;
+            if (a.logit_offset) logit = __fadd_rn(logit, a.logit_offset[e]);
+            sc[e] = logit;
+            if (a.exact_order) sc[a.E + e] = absum;
+            if (a.counter != nullptr && a.mode != 0) sc[2 * a.E + e] = sigmoid_ref(logit);
+        }
+    }
+}
+
+constexpr int kSelectWarps = 4;         // one selects and adds, three prepare products of a near-tie recomputation, each on a scheduler of its own
+constexpr int kSelectThreads = kSelectWarps * 32;
+
+__global__ void __launch_bounds__(kSelectThreads) router_select_kernel(RouterArgs a) {
     __shared__ TopKSmem sm;
     __shared__ __align__(16) float ring[kSeqRingFloats];
     if (threadIdx.x == 0) {
         pdl_trigger();
-        topk_smem_init(sm, kRouterWarps - 1);
+        topk_smem_init(sm, kSelectWarps - 1);
     }
     router_args_of_token(a, blockIdx.x);
     pdl_wait();   // the logits are the rows kernel's output
     __syncthreads();
-    router_finish(a, sm, ring, threadIdx.x, kRouterThreads, a.mode != 0, true, nullptr, nullptr);
+    router_finish(a, sm, ring, threadIdx.x, kSelectThreads, a.mode != 0, true, nullptr, nullptr);
 }
 
 template <class K, class... Args>
@@ -288,6 +422,17 @@ static int launch_router_pdl(K kernel, dim3 grid, int threads, size_t smem, cuda
     return (int)cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+template <int XD, int WD, int TB>
+static int launch_rows_batch_t(const RouterArgs& a, cudaStream_t st, int n_tokens) {
+    const size_t smem = kRowsPerCta * (size_t)a.H * (WD == W_F32 ? 4 : 2) + 16;
+    static const cudaError_t attr = cudaFuncSetAttribute(router_rows_batch_kernel<XD, WD, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget);
+    if (attr != cudaSuccess) return (int)attr;
+    // few experts leave SMs idle: then the token groups are spread over further CTAs, which read the rows again
+    const int gx = (a.E + kRowsPerCta - 1) / kRowsPerCta, groups = (n_tokens + TB - 1) / TB;
+    const int gy = max(1, min((groups + 1) / 2, sm_count() / gx));
+    return launch_router_pdl(router_rows_batch_kernel<XD, WD, TB>, dim3(gx, gy), kBatchThreads, smem, st, a, n_tokens);
+}
+
 // The rows-resident pair of launches; VIB3_ERR_UNSUPPORTED when the rows and two token buffers do not fit.
 template <int XD, int WD>
 static int launch_rows_t(const RouterArgs& a, cudaStream_t st, int n_tokens) {
@@ -299,9 +444,12 @@ static int launch_rows_t(const RouterArgs& a, cudaStream_t st, int n_tokens) {
     static const cudaError_t attr = cudaFuncSetAttribute(router_rows_kernel<XD, WD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget);
     if (attr != cudaSuccess) return (int)attr;
     const dim3 grid((a.E + kRowsPerCta - 1) / kRowsPerCta);
-    if (int e = launch_router_pdl(router_rows_kernel<XD, WD>, grid, kRowsThreads, smem, st, a, n_tokens, tok_chunk)) return e;
+    if (n_tokens > kBatchMinTokens) {
+        const int e = n_tokens <= kBatchWarps ? launch_rows_batch_t<XD, WD, 1>(a, st, n_tokens) : launch_rows_batch_t<XD, WD, 4>(a, st, n_tokens);
+        if (e != VIB3_OK) return e;
+    } else if (int e = launch_router_pdl(router_rows_kernel<XD, WD>, grid, kRowsThreads, smem, st, a, n_tokens, tok_chunk)) return e;
     if (a.counter == nullptr) return VIB3_OK;   // logits only
-    return launch_router_pdl(router_select_kernel, dim3(n_tokens), kRouterThreads, 0, st, a);
+    return launch_router_pdl(router_select_kernel, dim3(n_tokens), kSelectThreads, 0, st, a);
 }
 
 template <int XD, int WD>
