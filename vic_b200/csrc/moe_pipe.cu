@@ -56,7 +56,7 @@ struct RoutedSmem {
 };
 
 template <int NCH, bool ROUTED>
-__global__ void __maxnreg__(ROUTED ? 96 : 80) moe_gateup_pipe_kernel(MoeLayerArgs a, RouterArgs r, int nstages) {
+__global__ void __maxnreg__(ROUTED ? 104 : 80) moe_gateup_pipe_kernel(MoeLayerArgs a, RouterArgs r, int nstages) {
     using MATH = MathQ16;
     constexpr int kTileRows = gateup_tile_rows(NCH);         // row pairs per stage
     constexpr int kGroupWarps = kTileRows / kPairsPerWarp;   // warps that consume a stage

@@ -33,7 +33,7 @@
 // selection scores among the best k+1 are closer than a bound on the summation-order
 // difference, the near-tied experts' logits are recomputed with one sequential multiply-then-add
 // chain per expert (the CPU order) before the final selection (router_core.cuh).  This costs about
-// 26 microseconds and happens for a few percent of tokens.
+// 20 microseconds and happens for a few percent of tokens.
 #include "pipe_common.cuh"
 #include "router_core.cuh"
 
@@ -391,12 +391,182 @@ __global__ void __launch_bounds__(kBatchThreads) router_rows_batch_kernel(Router
     }
 }
 
-constexpr int kSelectWarps = 4;         // one selects and adds, three prepare products of a near-tie recomputation, each on a scheduler of its own
-constexpr int kSelectThreads = kSelectWarps * 32;
-
-__global__ void __launch_bounds__(kSelectThreads) router_select_kernel(RouterArgs a) {
+__global__ void __launch_bounds__(kRouterThreads) router_select_kernel(RouterArgs a) {
     __shared__ TopKSmem sm;
     __shared__ __align__(16) float ring[kSeqRingFloats];
+    if (threadIdx.x == 0) {
+        pdl_trigger();
+        topk_smem_init(sm, kRouterWarps - 1);
+    }
+    router_args_of_token(a, blockIdx.x);
+    pdl_wait();   // the logits are the rows kernel's output
+    __syncthreads();
+    router_finish(a, sm, ring, threadIdx.x, kRouterThreads, a.mode != 0, true, nullptr, nullptr);
+}
+
+// ── near-tie recomputation of a batched selection ────────────────────────────────────────────
+// Nearly every batched call has a token with near-tied experts, and the call lasts as long as its slowest token.  As
+// sequential_logits (router_core.cuh), but for up to eight experts side by side instead of four, with the helper
+// warps' operands requested before they wait for their half of the ring, and 16 products read while the 16 before are
+// added, other banks per lane.  7168 additions, Kimi shape: 26 us for up to eight candidates, there 29 us for four and
+// 47 for more.  A single token keeps the other one: its launch is cold code on the path to the expert kernels, and
+// with this one a host step took 2 us longer.
+constexpr int kSeqBatchCands = 8;
+constexpr int kSeqBatchBlock = 256;
+constexpr int kSeqBatchStride = kSeqBatchBlock + 4;
+constexpr int kSeqBatchRingFloats = kSeqBatchCands * 2 * kSeqBatchStride;
+
+// A helper warp of a recomputation (see sequential_logits_batch), whole 4-element items, aligned rows.
+template <int XD, int WD>
+__device__ __forceinline__ void seq_helper(const RouterArgs& a, TopKSmem& sm, float* ring, const int* cands, int nc, unsigned first, int nblocks,
+                                           int hw, int nh, int lane) {
+    using XT = typename XItem<XD>::T;
+    using WI = WItem<WD>;
+    constexpr int U = 4;   // items of a lane requested together
+    const int t_first = hw * 32 + lane, t_step = nh * 32;
+    XT xv[U];
+    typename WI::T wv[U];
+    constexpr int kItems = kSeqBatchBlock / 4;   // of a candidate and block: pair t is (candidate t / kItems, item t % kItems)
+    const int total = nc * kItems;
+    auto load4 = [&](int b, int t0) {
+        const int n4 = min(kSeqBatchBlock, a.H - b * kSeqBatchBlock) >> 2;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int t = t0 + u * t_step, i = t % kItems;
+            if (t < total && i < n4) {
+                xv[u] = __ldg(reinterpret_cast<const XT*>(a.x) + b * kItems + i);
+                wv[u] = WI::load(reinterpret_cast<const unsigned char*>(a.W) + (size_t)cands[t / kItems] * a.H * (WD == W_F32 ? 4 : 2), b * kItems + i);
+            }
+        }
+    };
+    load4(0, t_first);
+    for (int b = 0; b < nblocks; ++b) {
+        const unsigned gb = first + b;
+        const int half = gb & 1;
+        if (gb >= 2 && !seq_bar_wait(&sm.seq_empty[half], ((gb >> 1) - 1) & 1)) { sm.failed = 1; break; }
+        const int n4 = min(kSeqBatchBlock, a.H - b * kSeqBatchBlock) >> 2;
+        for (int t0 = t_first; t0 < total; t0 += t_step * U) {
+            if (t0 != t_first) load4(b, t0);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int t = t0 + u * t_step, i = t % kItems;
+                if (t < total && i < n4) {
+                    const float4 x = x_item<XD>(reinterpret_cast<const unsigned char*>(&xv[u]), 0), w = WI::cvt(wv[u]);
+                    *reinterpret_cast<float4*>(ring + (half * kSeqBatchCands + t / kItems) * kSeqBatchStride + 4 * i) =
+                        make_float4(__fmul_rn(x.x, w.x), __fmul_rn(x.y, w.y), __fmul_rn(x.z, w.z), __fmul_rn(x.w, w.w));
+                }
+            }
+        }
+        __syncwarp();
+        if (lane == 0) seq_bar_arrive(&sm.seq_full[half]);
+        if (b + 1 < nblocks) load4(b + 1, t_first);
+    }
+}
+
+__device__ __noinline__ static float sequential_logits_batch(const RouterArgs a, TopKSmem& sm, float* ring, const int* cands, int nc, int warp, int nwarps,
+                                                            int lane) {
+    const int nblocks = (a.H + kSeqBatchBlock - 1) / kSeqBatchBlock;
+    const unsigned first = sm.seq_blocks;  // (read before anybody advances it: the caller synchronised)
+    float acc = 0.f;
+    if (warp == 0) {
+        for (int b = 0; b < nblocks; ++b) {
+            const unsigned gb = first + b;
+            const int half = gb & 1;
+            if (!seq_bar_wait(&sm.seq_full[half], (gb >> 1) & 1)) { sm.failed = 1; break; }
+            if (lane < nc) {
+                const float* p = ring + (half * kSeqBatchCands + lane) * kSeqBatchStride;
+                const int n = min(kSeqBatchBlock, a.H - b * kSeqBatchBlock);
+                // two sets of 16 products: one is added while the other is read (past the block's end: its padding; not used)
+                float4 q[2][4];
+                auto load = [&](int set, int i) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) q[set][j] = *reinterpret_cast<const float4*>(p + min(i + 4 * j, kSeqBatchBlock));
+                };
+                auto add = [&](int set) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        acc = __fadd_rn(acc, q[set][j].x);
+                        acc = __fadd_rn(acc, q[set][j].y);
+                        acc = __fadd_rn(acc, q[set][j].z);
+                        acc = __fadd_rn(acc, q[set][j].w);
+                    }
+                };
+                int i = 0;
+                load(0, 0);
+                for (; i + 32 <= n; i += 32) {
+                    load(1, i + 16);
+                    add(0);
+                    load(0, i + 32);
+                    add(1);
+                }
+                for (; i < n; ++i) acc = __fadd_rn(acc, p[i]);
+            }
+            __syncwarp();
+            if (lane == 0) seq_bar_arrive(&sm.seq_empty[half]);
+        }
+    } else {
+        const int hw = warp - 1, nh = nwarps - 1;
+        if (a.H % 4 == 0 && ((uintptr_t)a.x & 15) == 0 && ((uintptr_t)a.W & 15) == 0) {
+            if (a.w_dtype == W_F32) {
+                if (a.x_dtype == X_F32) seq_helper<X_F32, W_F32>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
+                else if (a.x_dtype == X_F16) seq_helper<X_F16, W_F32>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
+                else seq_helper<X_BF16, W_F32>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
+            } else {
+                if (a.x_dtype == X_F32) seq_helper<X_F32, W_F16>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
+                else if (a.x_dtype == X_F16) seq_helper<X_F16, W_F16>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
+                else seq_helper<X_BF16, W_F16>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
+            }
+            return acc;
+        }
+        // rows that are not 16-byte aligned, or of odd length: element by element
+        const int t_first = hw * 32 + lane, t_step = nh * 32;
+        for (int b = 0; b < nblocks; ++b) {
+            const unsigned gb = first + b;
+            const int half = gb & 1;
+            if (gb >= 2 && !seq_bar_wait(&sm.seq_empty[half], ((gb >> 1) - 1) & 1)) { sm.failed = 1; break; }
+            const int n = min(kSeqBatchBlock, a.H - b * kSeqBatchBlock);
+            const int total = nc * n;
+            for (int t0 = t_first; t0 < total; t0 += t_step * 8) {
+                float xv[8], wv[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int t = t0 + u * t_step;
+                    const bool in = t < total;
+                    const int c = in ? t / n : 0, i = in ? t - c * n : 0;
+                    const int d = b * kSeqBatchBlock + i;
+                    xv[u] = in ? load_x_as_f32(a.x, a.x_dtype, d) : 0.f;
+                    wv[u] = in ? load_w(a.W, a.w_dtype, (size_t)cands[c] * a.H + d) : 0.f;
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int t = t0 + u * t_step;
+                    if (t < total) {
+                        const int c = t / n, i = t - c * n;
+                        ring[(half * kSeqBatchCands + c) * kSeqBatchStride + i] = __fmul_rn(xv[u], wv[u]);
+                    }
+                }
+            }
+            __syncwarp();
+            if (lane == 0) seq_bar_arrive(&sm.seq_full[half]);
+        }
+    }
+    return acc;
+}
+
+struct SeqBatch {
+    static constexpr int kCands = kSeqBatchCands, kBlock = kSeqBatchBlock;
+    static __device__ __forceinline__ float run(const RouterArgs& a, TopKSmem& sm, float* ring, const int* cands, int nc, int warp, int nwarps, int lane) {
+        return sequential_logits_batch(a, sm, ring, cands, nc, warp, nwarps, lane);
+    }
+};
+
+constexpr int kSelectWarps = 4;         // one selects and adds, three prepare products, each on a scheduler of its own
+constexpr int kSelectThreads = kSelectWarps * 32;
+
+// router_select_kernel for several tokens.
+__global__ void __launch_bounds__(kSelectThreads) router_select_batch_kernel(RouterArgs a) {
+    __shared__ TopKSmem sm;
+    __shared__ __align__(16) float ring[kSeqBatchRingFloats];
     if (threadIdx.x == 0) {
         pdl_trigger();
         topk_smem_init(sm, kSelectWarps - 1);
@@ -404,7 +574,7 @@ __global__ void __launch_bounds__(kSelectThreads) router_select_kernel(RouterArg
     router_args_of_token(a, blockIdx.x);
     pdl_wait();   // the logits are the rows kernel's output
     __syncthreads();
-    router_finish(a, sm, ring, threadIdx.x, kSelectThreads, a.mode != 0, true, nullptr, nullptr);
+    router_finish<SeqBatch>(a, sm, ring, threadIdx.x, kSelectThreads, a.mode != 0, true, nullptr, nullptr);
 }
 
 template <class K, class... Args>
@@ -449,7 +619,8 @@ static int launch_rows_t(const RouterArgs& a, cudaStream_t st, int n_tokens) {
         if (e != VIB3_OK) return e;
     } else if (int e = launch_router_pdl(router_rows_kernel<XD, WD>, grid, kRowsThreads, smem, st, a, n_tokens, tok_chunk)) return e;
     if (a.counter == nullptr) return VIB3_OK;   // logits only
-    return launch_router_pdl(router_select_kernel, dim3(n_tokens), kSelectThreads, 0, st, a);
+    if (n_tokens == 1) return launch_router_pdl(router_select_kernel, dim3(1), kRouterThreads, 0, st, a);
+    return launch_router_pdl(router_select_batch_kernel, dim3(n_tokens), kSelectThreads, 0, st, a);
 }
 
 template <int XD, int WD>

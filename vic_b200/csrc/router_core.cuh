@@ -10,9 +10,8 @@ namespace vib3 {
 constexpr int kRouterMaxExperts = 512;  // MAX_EXPERTS, src/core/types.rs:20
 constexpr int kRouterMaxTopK = 16;      // MAX_ACTIVE_EXPERTS, src/core/types.rs:26
 constexpr int kRouterXMax = 8192;       // widest activation vector staged in shared memory
-constexpr int kSeqCands = 8;            // near-tied experts recomputed side by side (more take further rounds)
-constexpr int kSeqBlock = 256;          // products per hand-over between the warps of a recomputation
-constexpr int kSeqStride = kSeqBlock + 4;  // of a candidate's products in the ring: eight lanes read eight of them, other banks each
+constexpr int kSeqCands = 4;            // near-tied experts recomputed side by side (more take further rounds)
+constexpr int kSeqBlock = 512;          // products per hand-over between the warps of a recomputation
 constexpr unsigned kRouterSpinLimit = 1u << 22;
 
 enum WDType : int { W_F16 = 0, W_F32 = 1 };
@@ -121,7 +120,7 @@ struct __align__(16) TopKSmem {
     unsigned long long seq_full[2], seq_empty[2];  // mbarriers of the recomputation's two ring halves
     unsigned seq_blocks;                           // blocks handed over so far (phase bookkeeping)
 };
-constexpr int kSeqRingFloats = kSeqCands * 2 * kSeqStride;  // 16.25 KB
+constexpr int kSeqRingFloats = kSeqCands * 2 * kSeqBlock;  // 16 KB
 
 // The reference kernel's reduction of an expert's 128 chain sums (kernels.cu:52-57, :682-705) when lane l
 // holds chains 4l .. 4l+3: its shfl_down tree over each group of 32 chains is, in this layout, three
@@ -227,63 +226,13 @@ __device__ __forceinline__ void topk_smem_init(TopKSmem& sm, int helper_warps) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
-// A helper warp of a recomputation (see sequential_logits), whole 4-element items, aligned rows.
-template <int XD, int WD>
-__device__ __forceinline__ void seq_helper(const RouterArgs& a, TopKSmem& sm, float* ring, const int* cands, int nc, unsigned first, int nblocks,
-                                           int hw, int nh, int lane) {
-    using XT = typename XItem<XD>::T;
-    using WI = WItem<WD>;
-    constexpr int U = 4;   // items of a lane requested together
-    const int t_first = hw * 32 + lane, t_step = nh * 32;
-    XT xv[U];
-    typename WI::T wv[U];
-    constexpr int kItems = kSeqBlock / 4;   // of a candidate and block: pair t is (candidate t / kItems, item t % kItems)
-    const int total = nc * kItems;
-    auto load4 = [&](int b, int t0) {
-        const int n4 = min(kSeqBlock, a.H - b * kSeqBlock) >> 2;
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int t = t0 + u * t_step, i = t % kItems;
-            if (t < total && i < n4) {
-                xv[u] = __ldg(reinterpret_cast<const XT*>(a.x) + b * kItems + i);
-                wv[u] = WI::load(reinterpret_cast<const unsigned char*>(a.W) + (size_t)cands[t / kItems] * a.H * (WD == W_F32 ? 4 : 2), b * kItems + i);
-            }
-        }
-    };
-    load4(0, t_first);
-    for (int b = 0; b < nblocks; ++b) {
-        const unsigned gb = first + b;
-        const int half = gb & 1;
-        if (gb >= 2 && !seq_bar_wait(&sm.seq_empty[half], ((gb >> 1) - 1) & 1)) { sm.failed = 1; break; }
-        const int n4 = min(kSeqBlock, a.H - b * kSeqBlock) >> 2;
-        for (int t0 = t_first; t0 < total; t0 += t_step * U) {
-            if (t0 != t_first) load4(b, t0);
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int t = t0 + u * t_step, i = t % kItems;
-                if (t < total && i < n4) {
-                    const float4 x = x_item<XD>(reinterpret_cast<const unsigned char*>(&xv[u]), 0), w = WI::cvt(wv[u]);
-                    *reinterpret_cast<float4*>(ring + (half * kSeqCands + t / kItems) * kSeqStride + 4 * i) =
-                        make_float4(__fmul_rn(x.x, w.x), __fmul_rn(x.y, w.y), __fmul_rn(x.z, w.z), __fmul_rn(x.w, w.w));
-                }
-            }
-        }
-        __syncwarp();
-        if (lane == 0) seq_bar_arrive(&sm.seq_full[half]);
-        if (b + 1 < nblocks) load4(b + 1, t_first);
-    }
-}
-
 // Logits of up to kSeqCands experts in the CPU router's order (kernels.rs:2346-2350): per expert a single
-// chain, multiply then add, d = 0 .. H-1.  The chain of dependent additions is the cost, whatever the number of candidates;
-// everything else hides under it: the group's first warp only adds — lane c owns candidate c's chain, and reads
-// 16 products while it adds the 16 before (other banks per lane) — and the other warps form the rounded products a
-// block of kSeqBlock ahead into a two-half ring in shared memory, from operands that they request before they wait for
-// the half.  The 7168 additions of the Kimi shape take 26 us for up to eight candidates; four at a time, with operands
-// requested after the wait and four lanes on one bank, it was 29 us for up to four and 47 for more.  `warp` is
-// the caller's index in the group, `nwarps` >= 2 its size.  Lane c < nc of warp 0 returns candidate c's sum.
-// (Not inlined: it runs for few tokens, and its registers would be everybody's.)
-__device__ __noinline__ static float sequential_logits(const RouterArgs& a, TopKSmem& sm, float* ring, const int* cands, int nc, int warp,
+// chain, multiply then add, d = 0 .. H-1.  The 7168 dependent additions of the Kimi shape are the cost
+// (about 18 us on B200, whatever the number of candidates); everything else hides under them: the group's
+// first warp only adds — lane c owns candidate c's chain — while the other warps form the rounded products
+// a block of kSeqBlock ahead into a two-half ring in shared memory.  `warp` is the caller's index in the
+// group, `nwarps` >= 2 its size.  Lane c < nc of warp 0 returns candidate c's sum.
+__device__ inline float sequential_logits(const RouterArgs& a, TopKSmem& sm, float* ring, const int* cands, int nc, int warp,
                                    int nwarps, int lane) {
     const int nblocks = (a.H + kSeqBlock - 1) / kSeqBlock;
     const unsigned first = sm.seq_blocks;  // (read before anybody advances it: the caller synchronised)
@@ -294,30 +243,20 @@ __device__ __noinline__ static float sequential_logits(const RouterArgs& a, TopK
             const int half = gb & 1;
             if (!seq_bar_wait(&sm.seq_full[half], (gb >> 1) & 1)) { sm.failed = 1; break; }
             if (lane < nc) {
-                const float* p = ring + (half * kSeqCands + lane) * kSeqStride;
+                const float* p = ring + (lane * 2 + half) * kSeqBlock;
                 const int n = min(kSeqBlock, a.H - b * kSeqBlock);
-                // two sets of 16 products: one is added while the other is read (past the block's end: its padding; not used)
-                float4 q[2][4];
-                auto load = [&](int set, int i) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) q[set][j] = *reinterpret_cast<const float4*>(p + min(i + 4 * j, kSeqBlock));
-                };
-                auto add = [&](int set) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        acc = __fadd_rn(acc, q[set][j].x);
-                        acc = __fadd_rn(acc, q[set][j].y);
-                        acc = __fadd_rn(acc, q[set][j].z);
-                        acc = __fadd_rn(acc, q[set][j].w);
-                    }
-                };
                 int i = 0;
-                load(0, 0);
                 for (; i + 32 <= n; i += 32) {
-                    load(1, i + 16);
-                    add(0);
-                    load(0, i + 32);
-                    add(1);
+                    float4 q[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) q[j] = *reinterpret_cast<const float4*>(p + i + 4 * j);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        acc = __fadd_rn(acc, q[j].x);
+                        acc = __fadd_rn(acc, q[j].y);
+                        acc = __fadd_rn(acc, q[j].z);
+                        acc = __fadd_rn(acc, q[j].w);
+                    }
                 }
                 for (; i < n; ++i) acc = __fadd_rn(acc, p[i]);
             }
@@ -326,43 +265,72 @@ __device__ __noinline__ static float sequential_logits(const RouterArgs& a, TopK
         }
     } else {
         const int hw = warp - 1, nh = nwarps - 1;
-        if (a.H % 4 == 0 && ((uintptr_t)a.x & 15) == 0 && ((uintptr_t)a.W & 15) == 0) {
-            if (a.w_dtype == W_F32) {
-                if (a.x_dtype == X_F32) seq_helper<X_F32, W_F32>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
-                else if (a.x_dtype == X_F16) seq_helper<X_F16, W_F32>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
-                else seq_helper<X_BF16, W_F32>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
-            } else {
-                if (a.x_dtype == X_F32) seq_helper<X_F32, W_F16>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
-                else if (a.x_dtype == X_F16) seq_helper<X_F16, W_F16>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
-                else seq_helper<X_BF16, W_F16>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
-            }
-            return acc;
-        }
-        // rows that are not 16-byte aligned, or of odd length: element by element
-        const int t_first = hw * 32 + lane, t_step = nh * 32;
         for (int b = 0; b < nblocks; ++b) {
             const unsigned gb = first + b;
             const int half = gb & 1;
             if (gb >= 2 && !seq_bar_wait(&sm.seq_empty[half], ((gb >> 1) - 1) & 1)) { sm.failed = 1; break; }
             const int n = min(kSeqBlock, a.H - b * kSeqBlock);
-            const int total = nc * n;
-            for (int t0 = t_first; t0 < total; t0 += t_step * 8) {
-                float xv[8], wv[8];
+            // (candidate, 4-element item) pairs of the block: one 16-byte (fp16 weights: 8-byte) load of the
+            // weights and one of the activations per item, all of a lane's items requested before any is used
+            // (one round trip per block); rows that are not 16-byte aligned take the scalar path
+            const bool vec = a.H % 4 == 0 && ((uintptr_t)a.x & 15) == 0 && ((uintptr_t)a.W & 15) == 0 && n % 4 == 0;
+            if (vec) {
+                const int n4 = n >> 2, total = nc * n4;
+                constexpr int U = 4;
+                for (int t0 = hw * 32 + lane; t0 < total; t0 += nh * 32 * U) {
+                    float4 xv[U], wv[U];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const int t = t0 + u * t_step;
-                    const bool in = t < total;
-                    const int c = in ? t / n : 0, i = in ? t - c * n : 0;
-                    const int d = b * kSeqBlock + i;
-                    xv[u] = in ? load_x_as_f32(a.x, a.x_dtype, d) : 0.f;
-                    wv[u] = in ? load_w(a.W, a.w_dtype, (size_t)cands[c] * a.H + d) : 0.f;
+                    for (int u = 0; u < U; ++u) {
+                        const int t = t0 + u * nh * 32;
+                        const bool in = t < total;
+                        const int c = in ? t / n4 : 0, i = in ? t - c * n4 : 0;
+                        const int item = (b * kSeqBlock >> 2) + i;
+                        if (a.x_dtype == X_F32) xv[u] = __ldg(reinterpret_cast<const float4*>(a.x) + item);
+                        else {
+                            const uint2 r2 = __ldg(reinterpret_cast<const uint2*>(a.x) + item);
+                            if (a.x_dtype == X_F16) {
+                                const __half2 p0 = *reinterpret_cast<const __half2*>(&r2.x), p1 = *reinterpret_cast<const __half2*>(&r2.y);
+                                xv[u] = make_float4(__low2float(p0), __high2float(p0), __low2float(p1), __high2float(p1));
+                            } else {
+                                xv[u] = make_float4(__uint_as_float(r2.x << 16), __uint_as_float(r2.x & 0xFFFF0000u),
+                                                    __uint_as_float(r2.y << 16), __uint_as_float(r2.y & 0xFFFF0000u));
+                            }
+                        }
+                        const size_t wi = ((size_t)cands[c] * a.H >> 2) + item;
+                        if (a.w_dtype == W_F32) wv[u] = __ldcg(reinterpret_cast<const float4*>(a.W) + wi);
+                        else wv[u] = WItem<W_F16>::cvt(__ldcg(reinterpret_cast<const uint2*>(a.W) + wi));
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const int t = t0 + u * nh * 32;
+                        if (t < total) {
+                            const int c = t / n4, i = t - c * n4;
+                            *reinterpret_cast<float4*>(ring + (c * 2 + half) * kSeqBlock + 4 * i) =
+                                make_float4(__fmul_rn(xv[u].x, wv[u].x), __fmul_rn(xv[u].y, wv[u].y), __fmul_rn(xv[u].z, wv[u].z),
+                                            __fmul_rn(xv[u].w, wv[u].w));
+                        }
+                    }
                 }
+            } else {
+                const int total = nc * n;
+                for (int t0 = (hw * 32 + lane); t0 < total; t0 += nh * 32 * 8) {
+                    float xv[8], wv[8];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const int t = t0 + u * t_step;
-                    if (t < total) {
-                        const int c = t / n, i = t - c * n;
-                        ring[(half * kSeqCands + c) * kSeqStride + i] = __fmul_rn(xv[u], wv[u]);
+                    for (int u = 0; u < 8; ++u) {
+                        const int t = t0 + u * nh * 32;
+                        const bool in = t < total;
+                        const int c = in ? t / n : 0, i = in ? t - c * n : 0;
+                        const int d = b * kSeqBlock + i;
+                        xv[u] = in ? load_x_as_f32(a.x, a.x_dtype, d) : 0.f;
+                        wv[u] = in ? load_w(a.W, a.w_dtype, (size_t)cands[c] * a.H + d) : 0.f;
+                    }
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        const int t = t0 + u * nh * 32;
+                        if (t < total) {
+                            const int c = t / n, i = t - c * n;
+                            ring[(c * 2 + half) * kSeqBlock + i] = __fmul_rn(xv[u], wv[u]);
+                        }
                     }
                 }
             }
@@ -372,6 +340,14 @@ __device__ __noinline__ static float sequential_logits(const RouterArgs& a, TopK
     }
     return acc;
 }
+
+// The recomputation that a single token's selection carries (see router_finish).
+struct SeqSingle {
+    static constexpr int kCands = kSeqCands, kBlock = kSeqBlock;
+    static __device__ __forceinline__ float run(const RouterArgs& a, TopKSmem& sm, float* ring, const int* cands, int nc, int warp, int nwarps, int lane) {
+        return sequential_logits(a, sm, ring, cands, nc, warp, nwarps, lane);
+    }
+};
 
 __device__ __forceinline__ void group_score(const RouterArgs& a, TopKSmem& sm, int tid, int nthreads) {
     for (int e = tid; e < a.E; e += nthreads) {
@@ -393,6 +369,8 @@ __device__ __forceinline__ void group_score(const RouterArgs& a, TopKSmem& sm, i
 // together; the group's first warp selects.  have_sig: a.scores[2E ..] already holds the sigmoid of every
 // logit.  write_global: store ids, weights (and recomputed logits) to a.out_ids / a.out_weights / a.scores.
 // ids_smem / w_smem (optional, shared memory, kRouterMaxTopK entries): receive the same results.
+// SEQ: how near-tied experts are recomputed.
+template <class SEQ = SeqSingle>
 __device__ inline void router_finish(const RouterArgs& a, TopKSmem& sm, float* ring, int tid, int nthreads, bool have_sig,
                               bool write_global, unsigned short* ids_smem, float* w_smem) {
     const int lane = tid & 31, warp = tid >> 5, nwarps = nthreads >> 5;
@@ -471,10 +449,10 @@ __device__ inline void router_finish(const RouterArgs& a, TopKSmem& sm, float* r
             if (cand) sm.cand[atomicAdd(&sm.ncand, 1)] = e;
         }
         group_sync(nthreads);
-        const int nblocks = (a.H + kSeqBlock - 1) / kSeqBlock;
-        for (int c0 = 0; c0 < sm.ncand; c0 += kSeqCands) {
-            const int nc = min(kSeqCands, sm.ncand - c0);
-            const float acc = sequential_logits(a, sm, ring, sm.cand + c0, nc, warp, nwarps, lane);
+        const int nblocks = (a.H + SEQ::kBlock - 1) / SEQ::kBlock;
+        for (int c0 = 0; c0 < sm.ncand; c0 += SEQ::kCands) {
+            const int nc = min(SEQ::kCands, sm.ncand - c0);
+            const float acc = SEQ::run(a, sm, ring, sm.cand + c0, nc, warp, nwarps, lane);
             if (warp == 0 && lane < nc) {
                 const int e = sm.cand[c0 + lane];
                 const float v = a.logit_offset ? __fadd_rn(acc, a.logit_offset[e]) : acc;
