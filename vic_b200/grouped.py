@@ -100,7 +100,7 @@ class GroupedDecoder:
             self.ids.stride(0) * 2, self.weights.data_ptr(), self.weights.stride(0) * 4, self.tables[layer],
             (self.shared_tables[layer] or None) if shared else None, 1.0, sh.pages_per_segment, lo, hi, out.data_ptr(),
             out.stride(0), int(accumulate),
-            self.status.data_ptr(), torch.cuda.current_stream().cuda_stream))
+            self.status.data_ptr(), kernels._stream()))
         return out
 
     def forward(self, layer: int, xs: torch.Tensor, out: Optional[torch.Tensor] = None, accumulate: bool = False,

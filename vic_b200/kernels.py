@@ -25,8 +25,14 @@ def _ptr(t) -> int:
     return t.data_ptr()
 
 
-def _stream(stream: Optional[int]) -> int:
-    return torch.cuda.current_stream().cuda_stream if stream is None else stream
+def _stream(stream: Optional[int] = None) -> int:
+    """The raw stream given, or torch's current one.  (torch.cuda.current_stream() builds a Stream object through six
+    layers of device look-ups: half of the host time of a per-page call.)"""
+    if stream is not None:
+        return stream
+    if not torch.cuda.is_initialized():
+        torch.cuda.init()
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def x_dtype_code(t: torch.Tensor) -> int:
