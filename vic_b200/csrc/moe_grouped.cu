@@ -21,7 +21,7 @@
 //      does not care about the order of K as long as both operands agree.
 //   D  fp32 in tensor memory, one accumulator per scale group of 32 columns (two MMAs of 16): scaling warps read a
 //      slab's accumulators with tcgen05.ld and add scale * D to their fp32 sums in registers, packed fp32 FMAs over
-//      as many token columns as the expert has (4, 8 or 16).  The scale costs one FMA per 32 weights and token
+//      as many token columns as the expert has (2, 4, 8 or 16).  The scale costs one FMA per 32 weights and token
 //      instead of one product per weight, and nothing is rounded between the codes and the fp32 sums.
 //      At the end of a tile: gate/up SiLU product rounded to fp16 as the batch-1 path does; down fp16 per (pair, row),
 //      combined per token in plan order by a last kernel, so that the result does not depend on scheduling.
@@ -167,10 +167,12 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
                  "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]),
                  "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
 }
-// N columns of this lane's row (N = 4, 8, 16); the values are there after tmem_ld_wait.
+// N columns of this lane's row (N = 2, 4, 8, 16); the values are there after tmem_ld_wait.
 template <int N>
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t* r) {
-    if constexpr (N == 4)
+    if constexpr (N == 2)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(taddr) : "memory");
+    else if constexpr (N == 4)
         asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
     else if constexpr (N == 8)
         asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -188,7 +190,7 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 // once the accumulators are in registers.
 template <int NE>
 __device__ __forceinline__ void scale_slab(uint32_t taddr, const uint4& sc, float2* acc, Bar release, int lane) {
-    constexpr int kBatch = NE == 4 ? 8 : NE == 8 ? 4 : 2;   // groups read together: 32 registers
+    constexpr int kBatch = NE <= 4 ? 8 : NE == 8 ? 4 : 2;   // groups read together: up to 32 registers
     const uint32_t sw[4] = {sc.x, sc.y, sc.z, sc.w};
 #pragma unroll
     for (int g0 = 0; g0 < 8; g0 += kBatch) {
@@ -562,6 +564,8 @@ __global__ void __launch_bounds__(kGrpThreads, 1) moe_grouped_kernel(const __gri
                         tc_fence_after();
                         if (!work) {
                             mbar_arrive_lane0(d_empty + team, lane);
+                        } else if (ntok <= 2) {
+                            scale_slab<2>(taddr, sc, acc, d_empty + team, lane);
                         } else if (ntok <= 4) {
                             scale_slab<4>(taddr, sc, acc, d_empty + team, lane);
                         } else if (ntok <= 8) {
