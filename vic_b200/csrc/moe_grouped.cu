@@ -233,7 +233,7 @@ __device__ __forceinline__ int perm8(int r) {
 }
 
 // One work unit: a 128-row A tile of one expert (gate/up: 64 gate rows and the same 64 up rows; down: 128 rows).
-// The units of a step are listed by build_units_kernel; unit u = (active expert u / tiles, tile u % tiles).
+// The units of a step are listed by build_units; unit u = (active expert u / tiles, tile u % tiles).
 struct __align__(16) Unit {
     int slot_a, slot_b;      // pool slots of the page(s); -1: page absent
     short row0;              // first row of the tile inside the page
@@ -790,11 +790,10 @@ struct BuildUnitsArgs {
     int* status;
 };
 
-__global__ void __launch_bounds__(256) build_units_kernel(BuildUnitsArgs b) {
-    pdl_wait();
+__device__ __forceinline__ void build_units(const BuildUnitsArgs& b, int block, int blocks) {
     const int per = b.tiles_gu + b.tiles_dn;
     const int total = b.work->n_active * per;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    for (int i = block * blockDim.x + threadIdx.x; i < total; i += blocks * blockDim.x) {
         const int ai = i / per, r = i - ai * per;
         const bool down = r >= b.tiles_gu;
         const int tile = down ? r - b.tiles_gu : r;
@@ -820,16 +819,14 @@ __global__ void __launch_bounds__(256) build_units_kernel(BuildUnitsArgs b) {
         u.pad2 = 0;
         (down ? b.units_dn : b.units_gu)[ai * (down ? b.tiles_dn : b.tiles_gu) + tile] = u;
     }
-    pdl_trigger();
 }
 
 // xg[p][perm(k)] = fp16(x[token(p)][k]): the tokens gathered in pair order, K order permuted per 8 columns.
-__global__ void __launch_bounds__(256) gather_tokens_kernel(const void* x, int x_dtype, int x_stride, const GroupedWork* work,
-                                                            const unsigned short* pair_token, __half* xg, int H) {
-    pdl_wait();
+__device__ __forceinline__ void gather_tokens(const void* x, int x_dtype, int x_stride, const GroupedWork* work, const unsigned short* pair_token, __half* xg,
+                                              int H, int block, int blocks) {
     const int n_pairs = work->n_pairs;
     const int items = H >> 3;
-    for (int p = blockIdx.x; p < n_pairs; p += gridDim.x) {
+    for (int p = block; p < n_pairs; p += blocks) {
         const unsigned char* row = reinterpret_cast<const unsigned char*>(x) + (size_t)pair_token[p] * x_stride;
         for (int i = threadIdx.x; i < items; i += blockDim.x) {
             float v[8];
@@ -846,6 +843,15 @@ __global__ void __launch_bounds__(256) gather_tokens_kernel(const void* x, int x
             reinterpret_cast<uint4*>(xg + (size_t)p * H)[i] = o;
         }
     }
+}
+
+// The two things that follow from the bucketing, in one launch: the first kUnitBlocks blocks list the units, the others
+// gather the tokens.  (One launch after the other they cost the chain of small kernels 3 us more.)
+constexpr int kUnitBlocks = 64;
+__global__ void __launch_bounds__(256) prepare_step_kernel(BuildUnitsArgs b, const void* x, int x_dtype, int x_stride, const unsigned short* pair_token, __half* xg, int H) {
+    pdl_wait();
+    if (blockIdx.x < kUnitBlocks) build_units(b, blockIdx.x, kUnitBlocks);
+    else gather_tokens(x, x_dtype, x_stride, b.work, pair_token, xg, H, blockIdx.x - kUnitBlocks, gridDim.x - kUnitBlocks);
     pdl_trigger();
 }
 
@@ -1124,17 +1130,14 @@ extern "C" int vib3_launch_moe_grouped_int4(void* handle, const void* x, int x_d
     g.pair_token = h->pair_token; g.status = status;
     int err = launch_pdl(group_pairs_kernel, dim3(1), 1024, 0, st, g);
     if (err) return err;
-    err = launch_pdl(gather_tokens_kernel, dim3(min(h->max_pairs, 2 * sm_count())), 256, 0, st, x, x_dtype, x_stride_bytes,
-                     (const GroupedWork*)h->work, (const unsigned short*)h->pair_token, h->xg, h->H);
-    if (err) return err;
-
     BuildUnitsArgs bu;
     bu.page_table = (const PageEntry*)page_table; bu.shared_pages = (const PageEntry*)shared_pages; bu.pool_base = h->pool_base;
     bu.work = h->work; bu.active = h->active; bu.counts = h->counts; bu.offsets = h->offsets; bu.units_gu = h->units_gu;
     bu.units_dn = h->units_dn; bu.tiles_gu = h->tiles_gu; bu.tiles_dn = h->tiles_dn; bu.tiles_per_page_gu = h->tiles_per_page_gu;
     bu.tiles_per_page_dn = h->tiles_per_page_dn; bu.E = h->E; bu.P = pages_per_segment; bu.rpp_gu = h->rpp_gu; bu.rpp_dn = h->rpp_dn;
     bu.status = status;
-    err = launch_pdl(build_units_kernel, dim3(64), 256, 0, st, bu);
+    err = launch_pdl(prepare_step_kernel, dim3(kUnitBlocks + min(h->max_pairs, 2 * sm_count())), 256, 0, st, bu, x, x_dtype, x_stride_bytes,
+                     (const unsigned short*)h->pair_token, h->xg, h->H);
     if (err) return err;
 
     GroupedArgs a;
