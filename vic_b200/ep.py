@@ -381,7 +381,7 @@ class ExpertParallelStack:
         self.ids_loc = torch.zeros(MAX_ACTIVE_EXPERTS, dtype=torch.int16, device=dev)
         self.w_loc = torch.zeros(MAX_ACTIVE_EXPERTS, dtype=torch.float32, device=dev)
         self.n_loc = torch.zeros(1, dtype=torch.int32, device=dev)
-        self.launches_per_layer = (4 if batch == 1 else 8) + (1 if world > 1 else 0)
+        self.launches_per_layer = (4 if batch == 1 else 7) + (1 if world > 1 else 0)
 
     def layer(self, l: int, prev: Optional[torch.Tensor]) -> torch.Tensor:
         from . import kernels as K
