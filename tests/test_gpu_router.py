@@ -237,3 +237,28 @@ def test_batched_logits_equal_single_token_logits(cuda_dev, E, H, ntok, xdt, wdt
         kernels.router_topk_batch(xs[t:t + 1], W, s1, None, None, i1, w1, k, 1, 2.5, True, 0, ws1)
         torch.cuda.synchronize()
         assert torch.equal(sc[t, :E], s1[0, :E]) and torch.equal(ids[t], i1[0]) and torch.equal(wt[t], w1[0]), t
+
+
+@pytest.mark.parametrize("H,offset", [(268, 0), (7172, 0), (520, 4), (268, 4)])
+def test_rows_that_a_bulk_copy_cannot_take(cuda_dev, oracle, H, offset):
+    """fp16 router rows that are not whole 16-byte units, or that start on an 8-byte boundary only, with fp32 tokens: they
+    belong to the direct kernel, for one token and for a batch."""
+    from vic_b200 import kernels
+    E, T, k = 7, 11, 3
+    g = torch.Generator(device="cpu").manual_seed(H + offset)
+    W = (0.05 * torch.randn(E, H, generator=g)).to(torch.float16)
+    Wd = torch.zeros(E * H + offset, dtype=torch.float16, device=cuda_dev)[offset:].view(E, H)
+    Wd.copy_(W)
+    assert Wd.data_ptr() % 16 == 2 * offset
+    xs = torch.randn(T, H, generator=g)
+    xs_d = xs.to(cuda_dev)
+    want = [oracle.router_logits(xs[t].numpy(), W.numpy(), oracle.ORDER_GPU128) for t in range(T)]
+    picks = [oracle.router(xs[t].numpy(), W.numpy(), k, 1, 2.5, True, None, oracle.ORDER_SEQUENTIAL)[0] for t in range(T)]
+    for n in (1, 2, T):
+        sc, ids = torch.zeros(n, 3 * E, device=cuda_dev), torch.zeros(n, 16, dtype=torch.int16, device=cuda_dev)
+        wt, ws = torch.zeros(n, 16, device=cuda_dev), torch.zeros(n, 4, dtype=torch.int32, device=cuda_dev)
+        kernels.router_topk_batch(xs_d[:n], Wd, sc, None, None, ids, wt, k, 1, 2.5, True, 0, ws)
+        sc_n = sc[:, :E].cpu().numpy()
+        assert all(np.array_equal(sc_n[t].view(np.uint32), want[t].view(np.uint32)) for t in range(n))
+        kernels.router_topk_batch(xs_d[:n], Wd, sc, None, None, ids, wt, k, 1, 2.5, True, 1, ws)
+        assert all(np.array_equal(ids[t, :k].cpu().numpy().view(np.uint16), picks[t]) for t in range(n))

@@ -14,7 +14,7 @@
 // a GPU.  The work split is different: ONE warp per expert row, lane l owns the four chains
 // 4l .. 4l+3, so that a lane's accesses are 16 bytes wide (fp32 weights) and a warp's cover 512
 // contiguous bytes.  Two implementations of that split:
-//   * rows-resident (the usual case: H a multiple of 8, aligned operands): a CTA brings three
+//   * rows-resident (the usual case: H a multiple of 8, 16-byte aligned operands): a CTA brings three
 //     expert rows into shared memory with one bulk copy each — requested before the kernel waits
 //     for the producer of the token, so the weights travel under the previous kernel's tail — and
 //     forms the logits of every token of the launch from there; a second launch (one CTA per token)
@@ -416,7 +416,8 @@ constexpr int kSeqBatchBlock = 256;
 constexpr int kSeqBatchStride = kSeqBatchBlock + 4;
 constexpr int kSeqBatchRingFloats = kSeqBatchCands * 2 * kSeqBatchStride;
 
-// A helper warp of a recomputation (see sequential_logits_batch), whole 4-element items, aligned rows.
+// A helper warp of a recomputation (see sequential_logits_batch): whole 4-element items of 16-byte aligned vectors and rows, which
+// is what the rows-resident launches are given (launch_rows_t).
 template <int XD, int WD>
 __device__ __forceinline__ void seq_helper(const RouterArgs& a, TopKSmem& sm, float* ring, const int* cands, int nc, unsigned first, int nblocks,
                                            int hw, int nh, int lane) {
@@ -506,48 +507,14 @@ __device__ __noinline__ static float sequential_logits_batch(const RouterArgs a,
         }
     } else {
         const int hw = warp - 1, nh = nwarps - 1;
-        if (a.H % 4 == 0 && ((uintptr_t)a.x & 15) == 0 && ((uintptr_t)a.W & 15) == 0) {
-            if (a.w_dtype == W_F32) {
-                if (a.x_dtype == X_F32) seq_helper<X_F32, W_F32>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
-                else if (a.x_dtype == X_F16) seq_helper<X_F16, W_F32>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
-                else seq_helper<X_BF16, W_F32>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
-            } else {
-                if (a.x_dtype == X_F32) seq_helper<X_F32, W_F16>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
-                else if (a.x_dtype == X_F16) seq_helper<X_F16, W_F16>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
-                else seq_helper<X_BF16, W_F16>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
-            }
-            return acc;
-        }
-        // rows that are not 16-byte aligned, or of odd length: element by element
-        const int t_first = hw * 32 + lane, t_step = nh * 32;
-        for (int b = 0; b < nblocks; ++b) {
-            const unsigned gb = first + b;
-            const int half = gb & 1;
-            if (gb >= 2 && !seq_bar_wait(&sm.seq_empty[half], ((gb >> 1) - 1) & 1)) { sm.failed = 1; break; }
-            const int n = min(kSeqBatchBlock, a.H - b * kSeqBatchBlock);
-            const int total = nc * n;
-            for (int t0 = t_first; t0 < total; t0 += t_step * 8) {
-                float xv[8], wv[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const int t = t0 + u * t_step;
-                    const bool in = t < total;
-                    const int c = in ? t / n : 0, i = in ? t - c * n : 0;
-                    const int d = b * kSeqBatchBlock + i;
-                    xv[u] = in ? load_x_as_f32(a.x, a.x_dtype, d) : 0.f;
-                    wv[u] = in ? load_w(a.W, a.w_dtype, (size_t)cands[c] * a.H + d) : 0.f;
-                }
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const int t = t0 + u * t_step;
-                    if (t < total) {
-                        const int c = t / n, i = t - c * n;
-                        ring[(half * kSeqBatchCands + c) * kSeqBatchStride + i] = __fmul_rn(xv[u], wv[u]);
-                    }
-                }
-            }
-            __syncwarp();
-            if (lane == 0) seq_bar_arrive(&sm.seq_full[half]);
+        if (a.w_dtype == W_F32) {
+            if (a.x_dtype == X_F32) seq_helper<X_F32, W_F32>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
+            else if (a.x_dtype == X_F16) seq_helper<X_F16, W_F32>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
+            else seq_helper<X_BF16, W_F32>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
+        } else {
+            if (a.x_dtype == X_F32) seq_helper<X_F32, W_F16>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
+            else if (a.x_dtype == X_F16) seq_helper<X_F16, W_F16>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
+            else seq_helper<X_BF16, W_F16>(a, sm, ring, cands, nc, first, nblocks, hw, nh, lane);
         }
     }
     return acc;
@@ -603,10 +570,13 @@ static int launch_rows_batch_t(const RouterArgs& a, cudaStream_t st, int n_token
     return launch_router_pdl(router_rows_batch_kernel<XD, WD, TB>, dim3(gx, gy), kBatchThreads, smem, st, a, n_tokens);
 }
 
-// The rows-resident pair of launches; VIB3_ERR_UNSUPPORTED when the rows and two token buffers do not fit.
+// The rows-resident pair of launches; VIB3_ERR_UNSUPPORTED (nothing launched: the direct kernel takes the call) when the rows
+// and two token buffers do not fit, or when a row is not what a bulk copy can take, whole 16-byte units from a 16-byte
+// boundary: fp32 tokens allow rows of H % 8 == 4 fp16 weights, and fp16 weights may start on an 8-byte boundary.
 template <int XD, int WD>
 static int launch_rows_t(const RouterArgs& a, cudaStream_t st, int n_tokens) {
     const size_t row_bytes = (size_t)a.H * (WD == W_F32 ? 4 : 2), xbytes = (size_t)a.H * (XD == X_F32 ? 4 : 2);
+    if (row_bytes % 16 || ((uintptr_t)a.W & 15)) return VIB3_ERR_UNSUPPORTED;
     int tok_chunk = n_tokens < kTokSlots ? n_tokens : kTokSlots;
     while (tok_chunk > 1 && kRowsPerCta * row_bytes + 2 * tok_chunk * xbytes + 64 > kSmemBudget) --tok_chunk;
     const size_t smem = kRowsPerCta * row_bytes + 2 * tok_chunk * xbytes + 64;
