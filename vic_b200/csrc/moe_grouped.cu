@@ -307,7 +307,8 @@ __global__ void __launch_bounds__(kGrpThreads, 1) moe_grouped_kernel(const __gri
     const Bar part_full = d_empty + 2;             // (one token group) team 1's partial sums are in exch
     const Bar up_full = part_full + 1;             // [team] (gate/up) the up rows' sums are in exch
     const Bar exch_free = up_full + 2;             // every scaling warp is through with this pass's exchange
-    const uint32_t tmem_slot = (exch_free + 1).addr;
+    const Bar mma_done = exch_free + 1;            // [issuer] (after a wait that ran out) all of the issuer's MMAs have completed
+    const uint32_t tmem_slot = (mma_done + kGrpMmaWarps).addr;
 
     const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
     const int K = DOWN ? a.I : a.H;
@@ -334,6 +335,7 @@ __global__ void __launch_bounds__(kGrpThreads, 1) moe_grouped_kernel(const __gri
         }
         mbar_init(part_full, 4);
         mbar_init(exch_free, 8);
+        for (int s = 0; s < kGrpMmaWarps; ++s) mbar_init(mma_done + s, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kGrpMmaWarp) {
@@ -474,7 +476,19 @@ __global__ void __launch_bounds__(kGrpThreads, 1) moe_grouped_kernel(const __gri
                 }
             }
         }
-        if (!ok && lane == 0) flag(a.status, kStatusTimeout);
+        // Nothing may be owed to this CTA when it leaves.  The last commits' arrivals on xempty and a_empty have no other waiter;
+        // after a wait that ran out, those phases may never complete, but this thread's own MMAs do, and until then they
+        // read shared memory and use tensor memory.
+        if (ok) {
+            for (int k = max(0, step - kGrpXStages); ok && k < step; ++k) ok = mbar_wait_grp(xempty + k % kGrpXStages, (k / kGrpXStages) & 1);
+            for (int k = max(0, it - 2); ok && k < it; ++k) ok = mbar_wait_grp(a_empty + (k & 1), (k >> 1) & 1);
+        }
+        if (!ok) {
+            if (elect_one()) umma_commit(mma_done + mw);
+            __syncwarp();
+            mbar_wait_grp(mma_done + mw, 0);
+            if (lane == 0) flag(a.status, kStatusTimeout);
+        }
     } else if (warp >= kGrpFirstConvWarp) {
         // ── converting warps: two teams of four take alternate slabs.  Row m = 32 (warp % 4) + lane of the A tile ──
         const int team = (warp - kGrpFirstConvWarp) >> 2;
@@ -563,6 +577,7 @@ __global__ void __launch_bounds__(kGrpThreads, 1) moe_grouped_kernel(const __gri
                         if (!ok) break;
                         tc_fence_after();
                         if (!work) {
+                            __syncwarp();   // (a lane still on its way out of the wait could otherwise miss the phase)
                             mbar_arrive_lane0(d_empty + team, lane);
                         } else if (ntok <= 2) {
                             scale_slab<2>(taddr, sc, acc, d_empty + team, lane);
@@ -1016,7 +1031,7 @@ int launch_pdl(K kernel, dim3 grid, int threads, size_t smem, cudaStream_t st, A
     return (int)cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-constexpr int kGrpBarriers = 2 * kGrpStages + 2 * kGrpXStages + 2 * kGrpScaleStages + 8 + 4 + 1;   // (+ the tensor memory address)
+constexpr int kGrpBarriers = 2 * kGrpStages + 2 * kGrpXStages + 2 * kGrpScaleStages + 8 + 4 + kGrpMmaWarps + 1;   // (+ the tensor memory address)
 constexpr size_t kGrpSmem = 1024 + (size_t)kGrpStages * kGrpCodeBytes + (size_t)kGrpXStages * kGrpXBytes + (size_t)kGrpScaleStages * kGrpScaleBytes +
                             128 * (kGrpMaxN + 1) * sizeof(float) + kGrpBarriers * sizeof(uint64_t);
 static_assert(kGrpSmem <= kSmemBudget, "shared memory of a CTA");
