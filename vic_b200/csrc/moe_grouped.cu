@@ -27,7 +27,7 @@
 //      combined per token in plan order by a last kernel, so that the result does not depend on scheduling.
 //
 // One elected thread per issuing warp issues MMAs; completion is tracked with tcgen05.commit on mbarriers.  Every wait is
-// bounded: a thread that gives up sets VIB3_STATUS_TIMEOUT and the CTA drains and frees its tensor memory.
+// bounded (about four seconds): a thread that gives up sets VIB3_STATUS_TIMEOUT and the CTA drains and frees its tensor memory.
 // No cluster launch, no multicast: every CTA fetches its own tiles.
 //
 // The path stays HBM-bound by construction: at 128 tokens the step has 90 GFLOP of tensor work (64 us at
@@ -102,12 +102,14 @@ struct Bar {
 };
 // The waits of this kernel: one look that does not suspend the warp, then suspending tries without a time limit of their
 // own.  A try with a suspend-time hint resumed later: with the hint the 32-token Kimi layer took 1025 us, without 983.
-// Bounded like every wait here; false when it gave up.
+// Bounded: a try whose phase does not complete comes back after 3.95 us (200 tries in a row: 790 us), so a wait gives up,
+// with false, after about four seconds.
+constexpr unsigned kGrpWaitTries = 1u << 20;
 __device__ __forceinline__ bool mbar_wait_grp(Bar bar, unsigned parity) {
     uint32_t ok;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(ok) : "r"(bar.addr), "r"(parity) : "memory");
-    for (unsigned it = 0; !ok && it < kSpinLimit; ++it)
+    for (unsigned it = 0; !ok && it < kGrpWaitTries; ++it)
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(ok) : "r"(bar.addr), "r"(parity) : "memory");
     return ok != 0;
@@ -393,12 +395,14 @@ __global__ void __launch_bounds__(kGrpThreads, 1) moe_grouped_kernel(const __gri
             }
         }
         if (!ok && lane == 0) flag(a.status, kStatusTimeout);
-        // drain: every issued copy must have landed before the CTA's shared memory goes away
+        // drain: every issued copy must have landed before the CTA's shared memory goes away (one wait that runs out ends
+        // the drain: four more seconds at most)
         if (lane == 0) {
-            for (int k = max(0, it - kGrpStages); k < it; ++k)
-                if (!mbar_wait_grp(full + (k % kGrpStages), (k / kGrpStages) & 1)) flag(a.status, kStatusTimeout);
-            for (int k = max(0, nchunk - kGrpScaleStages); k < nchunk; ++k)
-                if (!mbar_wait_grp(sfull + (k % kGrpScaleStages), (k / kGrpScaleStages) & 1)) flag(a.status, kStatusTimeout);
+            bool landed = true;
+            for (int k = max(0, it - kGrpStages); landed && k < it; ++k) landed = mbar_wait_grp(full + (k % kGrpStages), (k / kGrpStages) & 1);
+            for (int k = max(0, nchunk - kGrpScaleStages); landed && k < nchunk; ++k)
+                landed = mbar_wait_grp(sfull + (k % kGrpScaleStages), (k / kGrpScaleStages) & 1);
+            if (!landed) flag(a.status, kStatusTimeout);
         }
     } else if (warp == kGrpXWarp) {
         // ── TMA producer of the token ring: one copy per step (four K-major tiles of 64 columns) ──
@@ -427,9 +431,11 @@ __global__ void __launch_bounds__(kGrpThreads, 1) moe_grouped_kernel(const __gri
             }
         }
         if (!ok && lane == 0) flag(a.status, kStatusTimeout);
-        if (lane == 0)
-            for (int k = max(0, n - kGrpXStages); k < n; ++k)
-                if (!mbar_wait_grp(xfull + (k % kGrpXStages), (k / kGrpXStages) & 1)) flag(a.status, kStatusTimeout);
+        if (lane == 0) {
+            bool landed = true;
+            for (int k = max(0, n - kGrpXStages); landed && k < n; ++k) landed = mbar_wait_grp(xfull + (k % kGrpXStages), (k / kGrpXStages) & 1);
+            if (!landed) flag(a.status, kStatusTimeout);
+        }
     } else if (warp < kGrpFirstScaleWarp) {
         // ── MMA issuers: per step and scale group (32 columns, an accumulator of its own) two MMAs; the issuers share the groups ──
         const int mw = warp - kGrpMmaWarp;
