@@ -272,21 +272,26 @@ struct UnitWalk {
     }
 };
 
+// The halves of a token group's columns, as compile-time numbers.
+struct First { static constexpr int value = 0; };
+struct Second { static constexpr int value = 1; };
+
 // DOWN = false: act[pair][perm(row)] = f16(silu(f16(Wg x)) * f16(Wu x)); DOWN = true: y[pair][row] = f16(Wd act).
 //
 // What bounds it: not memory (the same walk without conversion, MMAs and scaling runs at 6.2 TB/s) and not the tensor pipe, but
 // the converting warps' instructions and the hand-overs between the roles.  Hence few warps (with 16 converting warps
 // the waits of all of them took more issue slots than their arithmetic gained: 1210 us against 1140), a whole slab per
 // hand-over (quarters: 1680 us), no scale product per weight, rolled conversion loops, operands that need no
-// per-lane moves (elect_one).  Kimi layer, experts' launches alone, before and now: 32 tokens (177 distinct experts,
-// 4.4 GB) 1203 -> 963 us = 4.55 TB/s; 8 tokens 306 -> 246 us; 128 tokens with skewed load 1317 -> 1128 us; Mixtral shape,
-// 50 tokens 294 -> 264 us.
+// per-lane moves (elect_one).  Experts' launches alone, with one fp16 product with the scale per weight (26 warps) and now: Kimi
+// layer, 32 tokens (177 distinct experts, 4.4 GB) 1201 -> 930 us = 4.7 TB/s; 8 tokens, even load, 430 -> 330 us; 128 tokens, skewed
+// load, 1350 -> 1162 us; Mixtral shape, 50 tokens, 292 -> 259 us.
 //
 // Every role walks the same sequence: units blockIdx.x, + gridDim.x, ...; per unit ceil(n_tok / 32) passes of one or two
 // token groups of 16; per pass nslab slabs of 256 columns; per slab a step for each token group.  `it` counts slabs (code
 // stage it % 8, A buffer and converting team it & 1), `step` steps (accumulator buffer and scaling team step & 1).  With
 // one token group the two scaling teams take alternate slabs of the same tokens and their sums meet at the end, with
-// two groups each team has its own.  A barrier is only ever waited for by roles that have seen its previous phase
+// two groups each team has its own (so the order of a token's fp32 sums depends on whether its expert has more than 16
+// tokens left, and on nothing else).  A barrier is only ever waited for by roles that have seen its previous phase
 // complete (a wait names its phase by one parity bit).
 template <bool DOWN>
 __global__ void __launch_bounds__(kGrpThreads, 1) moe_grouped_kernel(const __grid_constant__ GroupedMaps maps, GroupedArgs a) {
@@ -306,8 +311,8 @@ __global__ void __launch_bounds__(kGrpThreads, 1) moe_grouped_kernel(const __gri
     const Bar a_empty = a_full + 2;                // [it & 1] the MMAs that read it have completed
     const Bar d_full = a_empty + 2;                // [step & 1] the accumulators are complete
     const Bar d_empty = d_full + 2;                // [step & 1] the accumulators have been read
-    const Bar part_full = d_empty + 2;             // (one token group) team 1's partial sums are in exch
-    const Bar up_full = part_full + 1;             // [team] (gate/up) the up rows' sums are in exch
+    const Bar part_full = d_empty + 2;             // [team] (one token group) the team's sums of the other's columns are in exch
+    const Bar up_full = part_full + 2;             // [team] (gate/up) the up rows' sums are in exch
     const Bar exch_free = up_full + 2;             // every scaling warp is through with this pass's exchange
     const Bar mma_done = exch_free + 1;            // [issuer] (after a wait that ran out) all of the issuer's MMAs have completed
     const uint32_t tmem_slot = (mma_done + kGrpMmaWarps).addr;
@@ -334,8 +339,8 @@ __global__ void __launch_bounds__(kGrpThreads, 1) moe_grouped_kernel(const __gri
             mbar_init(d_full + s, kGrpMmaWarps);
             mbar_init(d_empty + s, 4);
             mbar_init(up_full + s, 2);
+            mbar_init(part_full + s, 4);
         }
-        mbar_init(part_full, 4);
         mbar_init(exch_free, 8);
         for (int s = 0; s < kGrpMmaWarps; ++s) mbar_init(mma_done + s, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -606,52 +611,65 @@ __global__ void __launch_bounds__(kGrpThreads, 1) moe_grouped_kernel(const __gri
                 }
                 if (pc > 0) ok = ok && mbar_wait_grp(exch_free, (pc - 1) & 1);
                 if (!ok) break;
+                // The ends of a pass, eight columns (a half) at a time.  With two token groups a team finishes both halves of its
+                // own.  With one, the teams' sums meet in shared memory: team 0 finishes the first half and, if there are more
+                // than eight tokens, team 1 the second.  While a team is busy here its accumulator buffer waits, which short units
+                // feel: 64 experts of 1024 x 4096, 12 tokens each, 199 us with all sixteen columns left to team 0, 186 so;
+                // Kimi layer, 8 tokens, 336 -> 330 us (loops of eight columns instead of sixteen).
+                const bool wide = ntok > 8;
                 float* ex = exch + m * (kGrpMaxN + 1);
-                bool store = true;
-                if (!two) {
-                    // one token group: the two teams' sums meet in shared memory; team 0 adds team 1's and stores
-                    if (team == 1) {
+                auto put = [&](float* to, auto half) {
+                    constexpr int h = decltype(half)::value;
 #pragma unroll
-                        for (int j = 0; j < kGrpMaxN / 2; ++j) {
-                            if (2 * j < ntok) {
-                                ex[2 * j] = acc[j].x;
-                                ex[2 * j + 1] = acc[j].y;
-                            }
-                        }
-                        __syncwarp();
-                        mbar_arrive_lane0(part_full, lane);
-                        store = false;
-                    } else {
-                        ok = mbar_wait_grp(part_full, n_part++ & 1);
-                        if (!ok) break;
-#pragma unroll
-                        for (int j = 0; j < kGrpMaxN / 2; ++j) {
-                            if (2 * j < ntok) {
-                                acc[j].x += ex[2 * j];
-                                acc[j].y += ex[2 * j + 1];
-                            }
+                    for (int j = 4 * h; j < 4 * h + 4; ++j) {
+                        if (2 * j < ntok) {
+                            to[2 * j] = acc[j].x;
+                            to[2 * j + 1] = acc[j].y;
                         }
                     }
+                };
+                auto take = [&](auto half) {
+                    constexpr int h = decltype(half)::value;
+#pragma unroll
+                    for (int j = 4 * h; j < 4 * h + 4; ++j) {
+                        if (2 * j < ntok) {
+                            acc[j].x += ex[2 * j];
+                            acc[j].y += ex[2 * j + 1];
+                        }
+                    }
+                };
+                if (!two) {
+                    if (team == 1) put(ex, First{});
+                    else if (wide) put(ex, Second{});
+                    if (team == 1 || wide) {
+                        __syncwarp();
+                        mbar_arrive_lane0(part_full + team, lane);
+                    }
+                    if (team == 0 || wide) ok = mbar_wait_grp(part_full + (team ^ 1), n_part++ & 1);
+                    if (!ok) break;
+                    if (team == 0) take(First{});
+                    else if (wide) take(Second{});
                 }
-                if (store && DOWN) {
+                const bool lo = two || team == 0, hi = wide && (two || team == 1);
+                if (DOWN) {
                     if (m < t.rows) {
                         __half* y = a.y + (size_t)(t.pair_off + t0) * a.H + t.mrow0 + m;
+                        auto store = [&](auto half) {
+                            constexpr int h = decltype(half)::value;
 #pragma unroll
-                        for (int j = 0; j < kGrpMaxN; ++j)
-                            if (j < ntok) y[(size_t)j * a.H] = __float2half_rn(j & 1 ? acc[j >> 1].y : acc[j >> 1].x);
+                            for (int j = 8 * h; j < 8 * h + 8; ++j)
+                                if (j < ntok) y[(size_t)j * a.H] = __float2half_rn(j & 1 ? acc[j >> 1].y : acc[j >> 1].x);
+                        };
+                        if (lo) store(First{});
+                        if (hi) store(Second{});
                     }
-                } else if (store) {
+                } else if (lo || hi) {
                     // the up half hands its values to the gate half of the same rows: through the second half of exch, or
                     // (two token groups) through the team's half
                     float* up = two ? exch + (team * 64 + (m & 63)) * (kGrpMaxN + 1) : exch + (64 + (m & 63)) * (kGrpMaxN + 1);
                     if (m >= 64) {
-#pragma unroll
-                        for (int j = 0; j < kGrpMaxN / 2; ++j) {
-                            if (2 * j < ntok) {
-                                up[2 * j] = acc[j].x;
-                                up[2 * j + 1] = acc[j].y;
-                            }
-                        }
+                        if (lo) put(up, First{});
+                        if (hi) put(up, Second{});
                         __syncwarp();
                         mbar_arrive_lane0(up_full + team, lane);
                     } else {
@@ -659,14 +677,19 @@ __global__ void __launch_bounds__(kGrpThreads, 1) moe_grouped_kernel(const __gri
                         if (!ok) break;
                         if (m < t.rows) {
                             __half* act = a.act + (size_t)(t.pair_off + t0) * a.I + perm8(t.mrow0 + m);
+                            auto store = [&](auto half) {
+                                constexpr int h = decltype(half)::value;
 #pragma unroll
-                            for (int j = 0; j < kGrpMaxN; ++j) {
-                                if (j < ntok) {
-                                    const float g16 = __half2float(__float2half_rn(j & 1 ? acc[j >> 1].y : acc[j >> 1].x));
-                                    const float u16 = __half2float(__float2half_rn(up[j]));
-                                    act[(size_t)j * a.I] = __float2half_rn(silu_mul_f32(g16, u16));
+                                for (int j = 8 * h; j < 8 * h + 8; ++j) {
+                                    if (j < ntok) {
+                                        const float g16 = __half2float(__float2half_rn(j & 1 ? acc[j >> 1].y : acc[j >> 1].x));
+                                        const float u16 = __half2float(__float2half_rn(up[j]));
+                                        act[(size_t)j * a.I] = __float2half_rn(silu_mul_f32(g16, u16));
+                                    }
                                 }
-                            }
+                            };
+                            if (lo) store(First{});
+                            if (hi) store(Second{});
                         }
                     }
                     ++n_up;
@@ -1037,7 +1060,7 @@ int launch_pdl(K kernel, dim3 grid, int threads, size_t smem, cudaStream_t st, A
     return (int)cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-constexpr int kGrpBarriers = 2 * kGrpStages + 2 * kGrpXStages + 2 * kGrpScaleStages + 8 + 4 + kGrpMmaWarps + 1;   // (+ the tensor memory address)
+constexpr int kGrpBarriers = 2 * kGrpStages + 2 * kGrpXStages + 2 * kGrpScaleStages + 8 + 5 + kGrpMmaWarps + 1;   // (+ the tensor memory address)
 constexpr size_t kGrpSmem = 1024 + (size_t)kGrpStages * kGrpCodeBytes + (size_t)kGrpXStages * kGrpXBytes + (size_t)kGrpScaleStages * kGrpScaleBytes +
                             128 * (kGrpMaxN + 1) * sizeof(float) + kGrpBarriers * sizeof(uint64_t);
 static_assert(kGrpSmem <= kSmemBudget, "shared memory of a CTA");
