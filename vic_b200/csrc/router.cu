@@ -267,8 +267,8 @@ __global__ void __launch_bounds__(kRowsThreads) router_rows_kernel(RouterArgs a,
 // shape; here it is 1 byte, and the multiply-adds (two per product: the sum, and the sum of magnitudes for the
 // near-tie bound, two at a time) come first.  The order of a logit's sum is the same (lane l owns chains 4l .. 4l + 3).
 // Whole batched router without recomputations, one (row, token) per warp -> here, bf16 tokens, Kimi shape: 16 tokens
-// 18.8 -> 16.5 us, 32: 33.2 -> 18.8, 128: 120.6 -> 53.6; 8 experts of 4096: 16 tokens 12.7 -> 10.7 us, 128: 79.4 -> 14.7.  Up to
-// 8 tokens the other kernel is the faster one (Kimi 11.5 against 14.2 us: too few warps have a token here); at 12 they tie.
+// 18.5 -> 15.7 us, 32: 33.0 -> 18.1, 128: 120.4 -> 53.0; 8 experts of 4096: 16 tokens 12.9 -> 10.5 us, 128: 80 -> 10.5.  Up to
+// 8 tokens the other kernel is the faster one (Kimi 11.1 against 14.1 us: too few warps have a token here).
 constexpr int kBatchWarps = 12;
 constexpr int kBatchThreads = kBatchWarps * 32;
 constexpr int kBatchMinTokens = 8;
@@ -305,7 +305,8 @@ __global__ void __launch_bounds__(kBatchThreads) router_rows_batch_kernel(Router
     if (a.hold_dependents && tid == 0) pdl_trigger();   // (see router_rows_kernel)
     const bool landed = mbar_wait(full, 0);
     const int n4 = a.H >> 2;
-    for (int t0 = (blockIdx.y * kBatchWarps + warp) * TB; t0 < n_tokens; t0 += gridDim.y * kBatchWarps * TB) {
+    // neighbouring groups of TB tokens go to different CTAs of the column: each has one as soon as there are as many groups as CTAs
+    for (int t0 = (warp * gridDim.y + blockIdx.y) * TB; t0 < n_tokens; t0 += gridDim.y * kBatchWarps * TB) {
         if (!landed) {
             if (lane == 0 && a.counter) a.counter[(size_t)t0 * a.counter_stride + 3] = 1u;
             continue;
@@ -564,9 +565,10 @@ static int launch_rows_batch_t(const RouterArgs& a, cudaStream_t st, int n_token
     const size_t smem = kRowsPerCta * (size_t)a.H * (WD == W_F32 ? 4 : 2) + 16;
     static const cudaError_t attr = cudaFuncSetAttribute(router_rows_batch_kernel<XD, WD, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget);
     if (attr != cudaSuccess) return (int)attr;
-    // few experts leave SMs idle: then the token groups are spread over further CTAs, which read the rows again
+    // few experts leave SMs idle: then the token groups are spread over further CTAs, which read the rows again (whole router, 50
+    // tokens: 8 experts x 4096 14.2 us with the groups left to the first CTA of a column, 10.5 spread; 64 x 2048 10.4 / 8.1)
     const int gx = (a.E + kRowsPerCta - 1) / kRowsPerCta, groups = (n_tokens + TB - 1) / TB;
-    const int gy = max(1, min((groups + 1) / 2, sm_count() / gx));
+    const int gy = max(1, min(groups, sm_count() / gx));
     return launch_router_pdl(router_rows_batch_kernel<XD, WD, TB>, dim3(gx, gy), kBatchThreads, smem, st, a, n_tokens);
 }
 
