@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(kRowsThreads) router_rows_kernel(RouterArgs a,
 // 8 tokens the other kernel is the faster one (Kimi 11.1 against 14.1 us: too few warps have a token here).
 constexpr int kBatchWarps = 12;
 constexpr int kBatchThreads = kBatchWarps * 32;
-constexpr int kBatchMinTokens = 8;
+constexpr int kRowsMaxTokens = 8;       // up to here router_rows_kernel takes the call, up to kBatchWarps sometimes (launch_rows_t)
 
 // acc += a b on both halves: two independent fp32 FMAs in one issue slot
 __device__ __forceinline__ void fma2(float2& acc, const float2& a, const float2& b) {
@@ -591,10 +591,19 @@ static int launch_rows_t(const RouterArgs& a, cudaStream_t st, int n_tokens) {
     static const cudaError_t attr = cudaFuncSetAttribute(router_rows_kernel<XD, WD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget);
     if (attr != cudaSuccess) return (int)attr;
     const dim3 grid((a.E + kRowsPerCta - 1) / kRowsPerCta);
-    if (n_tokens > kBatchMinTokens) {
-        const int e = n_tokens <= kBatchWarps ? launch_rows_batch_t<XD, WD, 1>(a, st, n_tokens) : launch_rows_batch_t<XD, WD, 4>(a, st, n_tokens);
-        if (e != VIB3_OK) return e;
-    } else if (int e = launch_router_pdl(router_rows_kernel<XD, WD>, grid, kRowsThreads, smem, st, a, n_tokens, tok_chunk)) return e;
+    // Up to 12 tokens a warp of the batched kernel has one token at most.  That pays where the tokens of a row triple are spread
+    // over several CTAs, or where they are fp32 (the other kernel stages them, twice the bytes), and loses once nearly every SM
+    // has rows of its own.  Whole router at 12 tokens, us, batched against not: 8 experts x 4096 8.8 / 10.5, 64 x 2048 6.7 / 9.1,
+    // 128 x 7168 13.2 / 14.6, 256 x 4096 (86 CTAs) 11.5 / 11.0 and at 9 tokens 10.9 / 12.7, 384 x 7168 (128 CTAs) 15.7 / 14.8 and at 9
+    // tokens 14.8 / 13.7, with fp32 tokens 16.3 / 21.9.  There fp16 weights with fp32 tokens do better with four tokens per warp:
+    // 16.3 us at 9 to 12 tokens, one per warp 17 to 18, not batched 15.6 to 19.5.
+    const bool few = n_tokens <= kBatchWarps, full = 4 * (int)grid.x > 3 * sm_count();
+    int e;
+    if (n_tokens <= kRowsMaxTokens || (few && full && XD != X_F32))
+        e = launch_router_pdl(router_rows_kernel<XD, WD>, grid, kRowsThreads, smem, st, a, n_tokens, tok_chunk);
+    else
+        e = few && !(full && WD == W_F16) ? launch_rows_batch_t<XD, WD, 1>(a, st, n_tokens) : launch_rows_batch_t<XD, WD, 4>(a, st, n_tokens);
+    if (e != VIB3_OK) return e;
     if (a.counter == nullptr) return VIB3_OK;   // logits only
     if (n_tokens == 1) return launch_router_pdl(router_select_kernel, dim3(1), kRouterThreads, 0, st, a);
     return launch_router_pdl(router_select_batch_kernel, dim3(n_tokens), kSelectThreads, 0, st, a);
