@@ -158,6 +158,7 @@ __global__ void __launch_bounds__(kRouterThreads) router_kernel(RouterArgs a) {
     if (tid == 0) topk_smem_init(sm, kRouterWarps - 1);
     __syncthreads();
     router_finish(a, sm, xbuf, tid, kRouterThreads, a.mode != 0, true, nullptr, nullptr);
+    if (tid == 32 && sm.failed) a.counter[3] = 1u;
     if (tid == 0) *a.counter = 0u;  // ready for the next launch
 }
 
@@ -408,6 +409,7 @@ __global__ void __launch_bounds__(kRouterThreads) router_select_kernel(RouterArg
     pdl_wait();   // the logits are the rows kernel's output
     __syncthreads();
     router_finish(a, sm, ring, threadIdx.x, kRouterThreads, a.mode != 0, true, nullptr, nullptr);
+    if (threadIdx.x == 32 && sm.failed) a.counter[3] = 1u;   // (a warp that is through: the first one still forms the weights)
 }
 
 // ── near-tie recomputation of a batched selection ────────────────────────────────────────────
@@ -536,8 +538,10 @@ struct SeqBatch {
 constexpr int kSelectWarps = 4;         // one selects and adds, three prepare products, each on a scheduler of its own
 constexpr int kSelectThreads = kSelectWarps * 32;
 
-// router_select_kernel for several tokens.
-__global__ void __launch_bounds__(kSelectThreads) router_select_batch_kernel(RouterArgs a) {
+// router_select_kernel for several tokens.  The logits were formed `group` tokens to a warp, which marks the first of them when its
+// wait runs out: here the mark reaches the others (in the logits kernel itself a loop over them cost 2 to 8 % of its time, by
+// another schedule of the arithmetic).
+__global__ void __launch_bounds__(kSelectThreads) router_select_batch_kernel(RouterArgs a, int group) {
     __shared__ TopKSmem sm;
     __shared__ __align__(16) float ring[kSeqBatchRingFloats];
     if (threadIdx.x == 0) {
@@ -548,6 +552,8 @@ __global__ void __launch_bounds__(kSelectThreads) router_select_batch_kernel(Rou
     pdl_wait();   // the logits are the rows kernel's output
     __syncthreads();
     router_finish<SeqBatch>(a, sm, ring, threadIdx.x, kSelectThreads, a.mode != 0, true, nullptr, nullptr);
+    const int nth = blockIdx.x % group;
+    if (threadIdx.x == 32 && (sm.failed || (nth && (a.counter - (size_t)nth * a.counter_stride)[3]))) a.counter[3] = 1u;
 }
 
 template <class K, class... Args>
@@ -598,15 +604,19 @@ static int launch_rows_t(const RouterArgs& a, cudaStream_t st, int n_tokens) {
     // tokens 14.8 / 13.7, with fp32 tokens 16.3 / 21.9.  There fp16 weights with fp32 tokens do better with four tokens per warp:
     // 16.3 us at 9 to 12 tokens, one per warp 17 to 18, not batched 15.6 to 19.5.
     const bool few = n_tokens <= kBatchWarps, full = 4 * (int)grid.x > 3 * sm_count();
-    int e;
-    if (n_tokens <= kRowsMaxTokens || (few && full && XD != X_F32))
+    int e, group = 1;   // tokens of a warp
+    if (n_tokens <= kRowsMaxTokens || (few && full && XD != X_F32)) {
         e = launch_router_pdl(router_rows_kernel<XD, WD>, grid, kRowsThreads, smem, st, a, n_tokens, tok_chunk);
-    else
-        e = few && !(full && WD == W_F16) ? launch_rows_batch_t<XD, WD, 1>(a, st, n_tokens) : launch_rows_batch_t<XD, WD, 4>(a, st, n_tokens);
+    } else if (few && !(full && WD == W_F16)) {
+        e = launch_rows_batch_t<XD, WD, 1>(a, st, n_tokens);
+    } else {
+        group = 4;
+        e = launch_rows_batch_t<XD, WD, 4>(a, st, n_tokens);
+    }
     if (e != VIB3_OK) return e;
     if (a.counter == nullptr) return VIB3_OK;   // logits only
     if (n_tokens == 1) return launch_router_pdl(router_select_kernel, dim3(1), kRouterThreads, 0, st, a);
-    return launch_router_pdl(router_select_batch_kernel, dim3(n_tokens), kSelectThreads, 0, st, a);
+    return launch_router_pdl(router_select_batch_kernel, dim3(n_tokens), kSelectThreads, 0, st, a, group);
 }
 
 template <int XD, int WD>
@@ -722,7 +732,7 @@ int make_router_args(const void* x, int x_dtype, const void* W, int w_dtype, flo
 // Extended launcher: one call (two launches chained by programmatic dependent launch; one on the direct path).  scores_buf holds 3E floats ([0, E) receives the logits, the rest is scratch);
 // workspace is four 32-bit words, zero before the first call: [0] is an arrival counter that every
 // call leaves at zero, [1] counts the near-tie recomputations done so far (diagnostics), [2] is used by
-// vib3_launch_moe_layer_routed_int4_paged, [3] is spare.
+// vib3_launch_moe_layer_routed_int4_paged, [3] is set when a bounded wait ran out.
 extern "C" int vib3_launch_router_topk_ex(const void* x, int x_dtype, const void* W, int w_dtype, float* scores_buf,
                                           const float* bias, const float* logit_offset, unsigned short* out_ids,
                                           float* out_weights,
