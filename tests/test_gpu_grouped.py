@@ -108,8 +108,9 @@ def test_grouped_accumulates_and_refuses_bad_arguments(cuda_dev):
 
 @pytest.mark.parametrize("H,I", [(768, 256), (256, 1280), (2304, 512)])
 def test_token_counts_and_slab_counts_at_the_edges(cuda_dev, oracle, H, I):
-    """Every token chooses every expert, so an expert has T tokens: the accumulator widths (4, 8, 16), one and two token
-    groups and several passes, over odd, single and partial slab counts of both projections."""
+    """Every token chooses every expert, so an expert has T tokens: the accumulator widths (2, 4, 8, 16), one and two token
+    groups, passes ended by one scaling team (up to 8 tokens) and by both, several passes, over odd, single and partial slab
+    counts of both projections."""
     from vic_b200.core_types import SCORING_SOFTMAX, MoeShape
     from vic_b200.grouped import GroupedDecoder
     from vic_b200.synth import build_synthetic_moe, synth_activation

@@ -218,10 +218,11 @@ def test_exact_order_bound_under_stress(cuda_dev, oracle, case):
 
 @pytest.mark.parametrize("E,H,ntok,xdt,wdt", [
     (5, 264, 9, torch.bfloat16, torch.float32), (3, 128, 12, torch.float16, torch.float16), (384, 1024, 13, torch.float32, torch.float32),
-    (7, 2056, 48, torch.bfloat16, torch.float16), (64, 520, 49, torch.float16, torch.float32), (16, 7168, 128, torch.bfloat16, torch.float32)])
+    (7, 2056, 48, torch.bfloat16, torch.float16), (64, 520, 49, torch.float16, torch.float32), (16, 7168, 128, torch.bfloat16, torch.float32),
+    (384, 264, 10, torch.bfloat16, torch.float32), (384, 264, 10, torch.float32, torch.float16), (340, 256, 12, torch.float16, torch.float16)])
 def test_batched_logits_equal_single_token_logits(cuda_dev, E, H, ntok, xdt, wdt):
-    """Token counts around the widths of the batched kernel, expert counts that leave rows of a CTA empty, row lengths that
-    leave lanes without an item: every logit is the single-token launch's bit for bit."""
+    """Token counts around the widths of the batched kernel, expert counts that leave rows of a CTA empty or few SMs to a second
+    CTA of the same rows, row lengths that leave lanes without an item: every logit is the single-token launch's bit for bit."""
     from vic_b200 import kernels
     g = torch.Generator(device=cuda_dev).manual_seed(E * H + ntok)
     W = (0.05 * torch.randn(E, H, generator=g, device=cuda_dev)).to(wdt)
@@ -262,3 +263,48 @@ def test_rows_that_a_bulk_copy_cannot_take(cuda_dev, oracle, H, offset):
         assert all(np.array_equal(sc_n[t].view(np.uint32), want[t].view(np.uint32)) for t in range(n))
         kernels.router_topk_batch(xs_d[:n], Wd, sc, None, None, ids, wt, k, 1, 2.5, True, 1, ws)
         assert all(np.array_equal(ids[t, :k].cpu().numpy().view(np.uint16), picks[t]) for t in range(n))
+
+
+@pytest.mark.parametrize("H,cands,T,xdt,wdt", [
+    (264, 2, 2, torch.bfloat16, torch.float32), (520, 9, 9, torch.float32, torch.float32), (520, 17, 13, torch.float16, torch.float32),
+    (776, 7, 13, torch.float32, torch.float16), (776, 8, 8, torch.bfloat16, torch.float16), (1016, 9, 2, torch.float16, torch.float16),
+    (7168, 17, 9, torch.bfloat16, torch.float32)])
+def test_batched_recomputation_of_near_ties(cuda_dev, oracle, H, cands, T, xdt, wdt):
+    """Every other token has `cands` near-tied experts at the top: one trip of the recomputation or several, last blocks that are
+    short, odd numbers of blocks.  The near-tied logits are then the CPU router's to the bit, all others the reference
+    kernel's, the selection is the CPU router's, and only those tokens count a recomputation."""
+    from vic_b200 import kernels
+    E, k = 40, 3
+    g = torch.Generator(device="cpu").manual_seed(H + cands)
+    base = torch.randn(H, generator=g)
+    W = torch.randn(E, H, generator=g) * (0.3 / H ** 0.5)
+    tied = torch.randperm(E, generator=g)[:cands].sort().values
+    W[tied] = 2 * base / base.dot(base)          # a logit of about 2; -2 for the other tokens
+    if wdt == torch.float32:                     # near ties and not only equal rows: differences below the sums' rounding
+        W[tied] *= 1 + 2.0 ** -22 * torch.randn(cands, H, generator=g)
+    W = W.to(wdt)
+    sign = torch.where(torch.arange(T) % 2 == 0, 1.0, -1.0)
+    xs = (sign[:, None] * base + 0.1 * torch.randn(T, H, generator=g)).to(xdt)
+    xs_n, W_n = xs.float().numpy(), W.numpy()
+
+    def run(x):
+        n = x.shape[0]
+        sc, ids = torch.zeros(n, 3 * E, device=cuda_dev), torch.zeros(n, 16, dtype=torch.int16, device=cuda_dev)
+        wt, ws = torch.zeros(n, 16, device=cuda_dev), torch.zeros(n, 4, dtype=torch.int32, device=cuda_dev)
+        kernels.router_topk_batch(x, Wd, sc, None, None, ids, wt, k, 1, 2.5, True, 1, ws)
+        return sc.cpu().numpy(), ids[:, :k].cpu().numpy().view(np.uint16), wt[:, :k].cpu().numpy(), ws.cpu().numpy()
+
+    Wd, xs_d = W.to(cuda_dev), xs.to(cuda_dev)
+    sc, ids, wt, ws = run(xs_d)
+    assert ws[:, 1].tolist() == [1 if t % 2 == 0 else 0 for t in range(T)] and not ws[:, [0, 2, 3]].any()
+    for t in range(T):
+        want = oracle.router_logits(xs_n[t], W_n, oracle.ORDER_GPU128)
+        if t % 2 == 0:
+            want[tied.numpy()] = oracle.router_logits(xs_n[t], W_n, oracle.ORDER_SEQUENTIAL)[tied.numpy()]
+        assert np.array_equal(sc[t, :E].view(np.uint32), want.view(np.uint32)), t
+        oi, ow, _ = oracle.router(xs_n[t], W_n, k, 1, 2.5, True, None, oracle.ORDER_SEQUENTIAL)
+        assert np.array_equal(ids[t], oi), t
+        assert np.allclose(wt[t], ow, rtol=2e-4), t
+        # sums of |x w|: a chain of at most H / 64 roundings and a tree of at most 8, in both forms
+        one = run(xs_d[t:t + 1])[0][0]
+        assert np.allclose(sc[t, E:2 * E], one[E:2 * E], rtol=(H / 64 + 8) * 2.0 ** -23, atol=0), t
