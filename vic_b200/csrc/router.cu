@@ -32,8 +32,8 @@
 // Bit-exact indices against the CPU router's sequential summation order: when any two adjacent
 // selection scores among the best k+1 are closer than a bound on the summation-order
 // difference, the near-tied experts' logits are recomputed with one sequential multiply-then-add
-// chain per expert (the CPU order) before the final selection (router_core.cuh).  This costs about
-// 20 microseconds and happens for a few percent of tokens.
+// chain per expert (the CPU order) before the final selection (router_core.cuh).  For two near-tied experts that costs
+// 25 to 30 microseconds (Kimi shape; more of them: router_core.cuh, and below for batches), and it happens for a few percent of tokens.
 #include "pipe_common.cuh"
 #include "router_core.cuh"
 
@@ -416,9 +416,9 @@ __global__ void __launch_bounds__(kRouterThreads) router_select_kernel(RouterArg
 // Nearly every batched call has a token with near-tied experts, and the call lasts as long as its slowest token.  As
 // sequential_logits (router_core.cuh), but for up to eight experts side by side instead of four, with the helper
 // warps' operands requested before they wait for their half of the ring, and 16 products read while the 16 before are
-// added, other banks per lane.  7168 additions, Kimi shape: 26 us for up to eight candidates, there 29 us for four and
-// 47 for more.  A single token keeps the other one: its launch is cold code on the path to the expert kernels, and
-// with this one a host step took 2 us longer.
+// added, other banks per lane.  Kimi shape (7168 additions), added to a call of 4 tokens: 25 us for two to five candidates, 28
+// for eight, 49 for nine; there, one token, 30 us for two, 47 for four, 85 for eight.  A single token keeps the other one: its
+// launch is cold code on the path to the expert kernels, and with this one a host step took 2 us longer.
 constexpr int kSeqBatchCands = 8;
 constexpr int kSeqBatchBlock = 256;
 constexpr int kSeqBatchStride = kSeqBatchBlock + 4;

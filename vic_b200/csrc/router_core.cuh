@@ -227,9 +227,9 @@ __device__ __forceinline__ void topk_smem_init(TopKSmem& sm, int helper_warps) {
 }
 
 // Logits of up to kSeqCands experts in the CPU router's order (kernels.rs:2346-2350): per expert a single
-// chain, multiply then add, d = 0 .. H-1.  The 7168 dependent additions of the Kimi shape are the cost
-// (about 18 us on B200, whatever the number of candidates); everything else hides under them: the group's
-// first warp only adds — lane c owns candidate c's chain — while the other warps form the rounded products
+// chain, multiply then add, d = 0 .. H-1.  The 7168 dependent additions of the Kimi shape and the preparation of
+// their products a block ahead are the cost (added to a one-token call, measured: two candidates 30 us, four 47, a further trip
+// 20 to 40): the group's first warp only adds — lane c owns candidate c's chain — while the other warps form the rounded products
 // a block of kSeqBlock ahead into a two-half ring in shared memory.  `warp` is the caller's index in the
 // group, `nwarps` >= 2 its size.  Lane c < nc of warp 0 returns candidate c's sum.
 __device__ inline float sequential_logits(const RouterArgs& a, TopKSmem& sm, float* ring, const int* cands, int nc, int warp,
